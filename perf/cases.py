@@ -38,35 +38,35 @@ VSINI, RV = (0.0, 300.0), (-150.0, 150.0)
 def listed():
     return [
         # the model of one label, as a notebook or an optimiser outside the framework asks for it (latency)
-        dict(name="model, one label", kind="model", grid="small", pixels=15000, labels=1, swarm="spread"),
+        dict(name="model one label", kind="model", grid="small", pixels=15000, labels=1, swarm="spread"),
         # models of a list of labels, returned whole (plots, training sets)
-        dict(name="models, 61 labels", kind="model", grid="survey", pixels=37501, labels=61, swarm="spread"),
+        dict(name="models 61 labels", kind="model", grid="survey", pixels=37501, labels=61, swarm="spread"),
         # one iteration of an outside sampler on one star: chi2 of a 40-particle swarm
-        dict(name="chi2, small swarm", kind="chi2", grid="small", pixels=15000, labels=40, swarm="near", continuum="chunk",
+        dict(name="chi2 small swarm", kind="chi2", grid="small", pixels=15000, labels=40, swarm="near", continuum="chunk",
              chunks=5, degree=8),
         # an early swarm or a coarse search: labels over many grid cubes
-        dict(name="chi2, spread labels", kind="chi2", grid="survey", pixels=37501, labels=2500, swarm="spread",
+        dict(name="chi2 spread labels", kind="chi2", grid="survey", pixels=37501, labels=2500, swarm="spread",
              continuum="chunk", chunks=8, degree=5),
         # a posterior or a late swarm: many labels within a cube, the longest spectrum (the largest case)
-        dict(name="chi2, contracted labels", kind="chi2", grid="survey", pixels=60000, labels=16001, swarm="contracted",
+        dict(name="chi2 contracted labels", kind="chi2", grid="survey", pixels=60000, labels=16001, swarm="contracted",
              continuum="chunk", chunks=8, degree=5),
         # wavelength-dependent resolution
-        dict(name="chi2, variable resolution", kind="chi2_variable", grid="survey", pixels=23456, labels=1000, swarm="near",
+        dict(name="chi2 variable resolution", kind="chi2_variable", grid="survey", pixels=23456, labels=1000, swarm="near",
              continuum="chunk", chunks=8, degree=5),
         # a design-matrix continuum on grids that carry the absolute flux
-        dict(name="chi2, linear continuum", kind="chi2", grid="factor", pixels=30007, labels=2048, swarm="contracted",
+        dict(name="chi2 linear continuum", kind="chi2", grid="factor", pixels=30007, labels=2048, swarm="contracted",
              continuum="linear", columns=40),
         # two stars in one spectrum
-        dict(name="chi2, binary", kind="binary", grid="small", pixels=15000, labels=160, swarm="near", continuum="chunk",
+        dict(name="chi2 binary", kind="binary", grid="small", pixels=15000, labels=160, swarm="near", continuum="chunk",
              chunks=5, degree=8),
         # one star, one swarm
-        dict(name="fit, one star", kind="fit", grid="small", stars=1, pixels_lo=15000, pixels_hi=15000, particles=40,
+        dict(name="fit one star", kind="fit", grid="small", stars=1, pixels_lo=15000, pixels_hi=15000, particles=40,
              iterations=10, swarm="spread", chunks=5, degree=8),
         # a batch of ragged spectra, swarms over the whole grid
-        dict(name="fits, spread swarms", kind="fit_many", grid="survey", stars=48, pixels_lo=10000, pixels_hi=60000,
+        dict(name="fits spread swarms", kind="fit_many", grid="survey", stars=48, pixels_lo=10000, pixels_hi=60000,
              particles=64, iterations=4, swarm="spread", chunks=8, degree=5),
         # a batch of ragged spectra refined within narrow ranges
-        dict(name="fits, narrow ranges", kind="fit_many", grid="survey", stars=128, pixels_lo=10000, pixels_hi=60000,
+        dict(name="fits narrow ranges", kind="fit_many", grid="survey", stars=128, pixels_lo=10000, pixels_hi=60000,
              particles=64, iterations=4, swarm="contracted", chunks=8, degree=5),
         # the server: more requests than slots, each with its own continuum settings (chunks 4-12, degree 3-8)
         dict(name="served fits", kind="served", grid="survey", stars=96, slots=40, pixels_lo=10000, pixels_hi=60000,
