@@ -17,6 +17,7 @@
 #include <cstdlib>
 
 #include "common.cuh"
+#include "device.cuh"
 #include "fft.cuh"
 #include "kernels.h"
 
@@ -27,7 +28,7 @@ __device__ __forceinline__ const float *final_row(const EvalBatch &b, const Eval
 }
 
 static int g_num_sms = 0;
-static int num_sms() {
+int num_sms() {
   if (!g_num_sms) {
     int dev;
     cudaGetDevice(&dev);
@@ -599,17 +600,6 @@ __device__ __forceinline__ void cp_async16(float *smem, const float *gmem, bool 
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-// Bulk prefetch of floats [lo, hi) of a row into L2 (one instruction, issued
-// by one thread; a hint, nothing waits for it).  The row must start on a
-// 16-byte boundary and hold hi rounded up to 4 floats.
-__device__ __forceinline__ void prefetch_row_l2(const float *row, int lo, int hi) {
-  lo &= ~3;
-  hi = (hi + 3) & ~3;
-  if (hi <= lo) return;
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(row + lo), "r"((unsigned)(hi - lo) * 4u)
-               : "memory");
-}
 
 struct BroadenItem {
   int e, pair, m, hg, V, s0, s1, j0, j1;
@@ -1456,13 +1446,6 @@ void launch_copy_broadened(const DevGrid &G, const EvalBatch &b, float *out, cud
 
 // ------------------------------------------------------------------ chi2
 constexpr int CT = 256, CW = CT / 32;
-// pixels per lane whose loads the chunk kernels issue together: 8 up to
-// degree 5 (the Legendre values of 8 pixels fit the 64 registers of 4 CTAs
-// per SM), 4 above
-template <int K>
-__host__ __device__ constexpr int chunk_cu() {
-  return K <= 6 ? 8 : 4;
-}
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -1536,36 +1519,11 @@ __device__ __forceinline__ double block_sum(double v, double (*ws)[MAX_P1]) {
   return r;
 }
 
-// Legendre P_0..P_{K-1} at x (f32, the host Gram uses the same recurrence)
-template <int K>
-__device__ __forceinline__ void legendre(float x, float (&P)[K]) {
-  P[0] = 1.0f;
-  if (K > 1) P[1] = x;
-#pragma unroll
-  for (int k = 1; k + 1 < K; k++) P[k + 1] = leg_step(leg_a(k), leg_c(k), x, P[k], P[k - 1]);
-}
-
-template <int K>
-__device__ __forceinline__ float poly_eval(const float *coef, float x) {
-  float P[K];
-  legendre<K>(x, P);
-  float s = 0.0f;
-#pragma unroll
-  for (int k = 0; k < K; k++) s = fmaf(coef[k], P[k], s);
-  return s;
-}
-
 __device__ __forceinline__ void write_result(const EvalBatch &b, int e, double chi2, int status) {
   if (threadIdx.x == 0) {
     b.cost[e] = status ? __longlong_as_double(0x7FF8000000000000ll) : chi2;
     b.status[e] = status;
   }
-}
-
-// model at the observed pixels of evaluation e
-__device__ __forceinline__ const float *model_row(const EvalBatch &b, const EvalPrep &P, int e) {
-  if (b.given) return b.given + (size_t)e * b.given_stride;
-  return (P.mobs_in_b ? b.bufB : b.bufA) + (size_t)e * b.stride;
 }
 
 // Evaluations that k_broaden did not resample: the model at the observed
@@ -1584,252 +1542,6 @@ void launch_resample_obs(const DevGrid &G, const EvalBatch &b, cudaStream_t s) {
   dim3 grid(b.E, 8);
   k_resample_obs<<<grid, 256, 0, s>>>(G, b);
   count_launch();
-}
-
-// ChunkFitter::fit_continuum (continuum_fitting.rs:382-396), one warp per
-// (evaluation, chunk): the unweighted least-squares polynomial of
-// flux/model over the chunk (216-226) is the projection onto the chunk's
-// polynomial space; it is solved here in a Legendre basis with the FP64
-// Cholesky factor of its Gram matrix (the same space as the reference's
-// monomial SVD, far better conditioned).  A lane sums the products
-// P_k(x) y of its CU pixels in f32 and adds that partial to its running
-// FP64 moment: one f32 -> f64 conversion per moment per CU pixels instead of
-// one per pixel (the conversions share the narrow XU pipe with the
-// division's reciprocal), and a short FP64 dependency chain.
-// K = polynomial order + 1 (one instantiation per order present).  A warp
-// walks the whole chunk (no block barriers), so the loads of many chunks
-// are in flight per SM.
-// Moments of chunk c walked by one warp; lane 0 then solves G a = z with the
-// chunk's FP64 Cholesky factor, leaving the Legendre coefficients in a[0..K)
-// (and the reference's parameters in b.params when requested).
-template <int K>
-__device__ __forceinline__ void chunk_solve_warp(const EvalBatch &b, const DevStar &st, const float *mod, int e,
-                                                 int c, int lane, double *a) {
-  const float *flux = st.flux;
-  const int lo = st.cstart[c], hi = st.cstop[c], prev = c > 0 ? st.cstop[c - 1] : -1;
-  if (lane == 0 && !b.given) prefetch_row_l2(mod, lo, hi);  // the walk below then reads from L2
-  constexpr int CU = chunk_cu<K>();
-  double z[K];
-#pragma unroll
-  for (int k = 0; k < K; k++) z[k] = 0.0;
-  // pixels [a0, a1) with chunk coordinates xs (the upper-chunk coordinate
-  // below the previous chunk's stop); loads of CU pixels are issued before
-  // any arithmetic on them
-  auto walk = [&](int a0, int a1, const float *__restrict__ xs) {
-    for (int i0 = a0 + lane; i0 < a1; i0 += 32 * CU) {
-      float fl[CU], md[CU], xf[CU];
-#pragma unroll
-      for (int u = 0; u < CU; u++) {
-        const int i = min(i0 + 32 * u, a1 - 1);
-        fl[u] = flux[i];
-        md[u] = mod[i];
-        xf[u] = xs[i];
-      }
-      float zp[K];
-#pragma unroll
-      for (int k = 0; k < K; k++) zp[k] = 0.0f;
-#pragma unroll
-      for (int u = 0; u < CU; u++) {
-        if (i0 + 32 * u < a1) {
-          // flux / model as x * rcp(y) (at most 2 ulp; the moments are sums
-          // of thousands of such terms, accumulated in FP64)
-          const float y = __fdividef(fl[u], md[u]);
-          float Pk[K];
-          legendre<K>(xf[u], Pk);
-#pragma unroll
-          for (int k = 0; k < K; k++) zp[k] = fmaf(Pk[k], y, zp[k]);
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < K; k++) z[k] += (double)zp[k];
-    }
-  };
-  const int split = c > 0 ? min(max(prev, lo), hi) : lo;
-  walk(lo, split, st.xb);
-  walk(split, hi, st.xa);
-#pragma unroll
-  for (int k = 0; k < K; k++) {
-    const double t = warp_sum(z[k]);
-    if (lane == 0) a[k] = t;
-  }
-  if (lane == 0) {  // FP64 Cholesky solve G a = z, in place
-    const double *L = st.chol + (size_t)c * K * K;
-    for (int k = 0; k < K; k++) {
-      double t = a[k];
-      for (int j = 0; j < k; j++) t -= L[k * K + j] * a[j];
-      a[k] = t / L[k * K + k];
-    }
-    for (int k = K - 1; k >= 0; k--) {
-      double t = a[k];
-      for (int j = k + 1; j < K; j++) t -= L[j * K + k] * a[j];
-      a[k] = t / L[k * K + k];
-    }
-    if (b.params) {
-      double *par = b.params + (size_t)e * b.param_stride + c * K;
-      for (int k = 0; k < K; k++) par[k] = a[k];
-    }
-  }
-}
-
-// Monomial coefficients of the Legendre polynomials, T[k][j] = coefficient
-// of x^j in P_k, from (k + 1) P_{k+1} = (2k + 1) x P_k - k P_{k-1} (dyadic
-// rationals, exact in double up to degree 15).
-struct LegMono {
-  double c[MAX_P1][MAX_P1];
-};
-constexpr LegMono make_leg_mono() {
-  LegMono t{};
-  t.c[0][0] = 1.0;
-  t.c[1][1] = 1.0;
-  for (int k = 1; k + 1 < MAX_P1; k++)
-    for (int j = 0; j < MAX_P1; j++)
-      t.c[k + 1][j] = ((2 * k + 1) * (j > 0 ? t.c[k][j - 1] : 0.0) - k * t.c[k - 1][j]) / (k + 1);
-  return t;
-}
-__constant__ LegMono c_leg_mono = make_leg_mono();
-
-// the chunk polynomial sum_k a_k P_k(x) as monomial coefficients (FP64),
-// rounded to f32 for Horner evaluation
-template <int K>
-__device__ __forceinline__ void legendre_to_monomial(const double *a, float *m) {
-  for (int j = 0; j < K; j++) {
-    double s = 0.0;
-    for (int k = j; k < K; k++) s = fma(a[k], c_leg_mono.c[k][j], s);
-    m[j] = (float)s;
-  }
-}
-
-template <int K>
-__device__ __forceinline__ float horner(const float (&a)[K], float x) {
-  float p = a[K - 1];
-#pragma unroll
-  for (int j = K - 2; j >= 0; j--) p = fmaf(p, x, a[j]);
-  return p;
-}
-
-// chi2 section of chunk c (continuum_fitting.rs:280-360) walked by one
-// warp: chunk 0 alone on [50, start_1); chunk c >= 1 blended with chunk
-// c - 1 (sin^2 factor) on [start_c, stop_{c-1}), then alone up to
-// start_{c+1} (N - 50 for the last).  A lane adds the terms of the pixels
-// it loads together in f32 and those partials in FP64; the warp's sum is
-// returned to lane 0.
-template <int K>
-__device__ __forceinline__ double chunk_resid_warp(const DevStar &st, const float *mod, int c, int lane,
-                                                   const float (&cc)[K], const float (&cp)[K]) {
-  const int N = st.n_obs, nc = st.n_chunks;
-  const float *flux = st.flux, *var = st.var;
-  double acc = 0.0;
-  constexpr int CU = chunk_cu<K>();
-  // [lo, hi) with chunk c alone; loads of CU pixels before their arithmetic
-  auto alone = [&](int lo, int hi) {
-    for (int i0 = lo + lane; i0 < hi; i0 += 32 * CU) {
-      float fl[CU], md[CU], vr[CU], xa[CU];
-#pragma unroll
-      for (int u = 0; u < CU; u++) {
-        const int i = min(i0 + 32 * u, hi - 1);
-        fl[u] = flux[i];
-        md[u] = mod[i];
-        vr[u] = var[i];
-        xa[u] = st.xa[i];
-      }
-      float part = 0.0f;  // the lane's CU terms in f32, then one FP64 add
-#pragma unroll
-      for (int u = 0; u < CU; u++) {
-        if (i0 + 32 * u < hi) {
-          const float p = horner<K>(cc, xa[u]);
-          const float r = fl[u] - p * md[u];
-          part += __fdividef(r * r, vr[u]);
-        }
-      }
-      acc += (double)part;
-    }
-  };
-  if (c == 0) {
-    alone(50, st.cstart[1]);
-  } else {
-    const int s0 = st.cstart[c], sp = st.cstop[c - 1];
-    const int nx = c == nc - 1 ? N - 50 : st.cstart[c + 1];
-    for (int i0 = s0 + lane; i0 < sp; i0 += 32 * 2) {  // overlap: blend previous and current
-      float fl[2], md[2], vr[2], xa[2], xb[2], fc[2];
-#pragma unroll
-      for (int u = 0; u < 2; u++) {
-        const int i = min(i0 + 32 * u, sp - 1);
-        fl[u] = flux[i];
-        md[u] = mod[i];
-        vr[u] = var[i];
-        xa[u] = st.xa[i];
-        xb[u] = st.xb[i];
-        fc[u] = st.fac[i];
-      }
-      float part = 0.0f;
-#pragma unroll
-      for (int u = 0; u < 2; u++) {
-        if (i0 + 32 * u < sp) {
-          const float pv = horner<K>(cp, xa[u]);
-          const float cu = horner<K>(cc, xb[u]);
-          const float p = pv * fc[u] + cu * (1.0f - fc[u]);
-          const float r = fl[u] - p * md[u];
-          part += __fdividef(r * r, vr[u]);
-        }
-      }
-      acc += (double)part;
-    }
-    alone(sp, nx);
-  }
-  return warp_sum(acc);
-}
-
-// ChunkFitter::fit_continuum + compute_chi2_from_chunks
-// (continuum_fitting.rs:216-226, 280-360, 382-396) for one evaluation per
-// CTA: warp w takes chunks w, w + 8, ...  First every chunk's moments and
-// FP64 solve: the unweighted least-squares polynomial of flux/model over
-// the chunk is the projection onto the chunk's polynomial space, solved here
-// in a Legendre basis with the Cholesky factor of its Gram matrix (the same
-// space as the reference's monomial SVD, far better conditioned).  After a
-// CTA barrier every chunk section's chi2 from the coefficients in shared
-// memory, reading the model row a second time while it is still in L2;
-// then the sections added in chunk order in FP64 / (N - 100).  Errors give
-// NaN with the evaluation's status.  K = polynomial order + 1 (one
-// instantiation per order present; other orders return at once).
-template <int K>
-__global__ void __launch_bounds__(CT, K <= 8 ? 4 : 2) k_chunk_fit(EvalBatch b) {
-  __shared__ double zs[MAX_CHUNKS][MAX_P1];
-  __shared__ float cfs[MAX_CHUNKS][MAX_P1];
-  __shared__ double part[MAX_CHUNKS];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int e = blockIdx.x;
-  const EvalPrep &P = b.prep[e];
-  const DevStar &st = b.stars[P.star];
-  if (st.cont_kind != CONT_CHUNK || st.p1 != K) return;
-  int status = P.status;
-  if (!status && st.cont_bad) status = S_CONTINUUM;
-  if (status) {
-    write_result(b, e, 0.0, status);
-    return;
-  }
-  const float *mod = model_row(b, P, e);
-  const int nc = st.n_chunks;
-  for (int c = warp; c < nc; c += CW) {
-    chunk_solve_warp<K>(b, st, mod, e, c, lane, zs[c]);
-    if (lane == 0) legendre_to_monomial<K>(zs[c], cfs[c]);
-  }
-  __syncthreads();
-  for (int c = warp; c < nc; c += CW) {
-    float cc[K], cp[K];
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-      cc[k] = cfs[c][k];
-      cp[k] = c > 0 ? cfs[c - 1][k] : 0.0f;
-    }
-    const double acc = chunk_resid_warp<K>(st, mod, c, lane, cc, cp);
-    if (lane == 0) part[c] = acc;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double chi2 = 0.0;
-    for (int c = 0; c < nc; c++) chi2 += part[c];
-    write_result(b, e, chi2 / (double)(st.n_obs - 100), 0);
-  }
 }
 
 // LinearModelFitter (continuum_fitting.rs:68-95): projection onto the design
@@ -1907,35 +1619,11 @@ __global__ void __launch_bounds__(CT) k_chi2_other(DevGrid G, EvalBatch b) {
   write_result(b, e, chi2, 0);
 }
 
-template <int K>
-static void launch_chunk(const EvalBatch &b, cudaStream_t s) {
-  k_chunk_fit<K><<<b.E, CT, 0, s>>>(b);
-  count_launch();
-}
-
 // chi2 of every evaluation from the model at its observed pixels
 // (model_row: resampled by k_broaden / k_resample_obs, or given)
 void launch_chi2(const DevGrid &G, const EvalBatch &b, cudaStream_t s) {
   if (b.E <= 0) return;
-  const uint32_t m = b.chunk_p1_mask;
-  if (m && b.max_chunks > 0) {
-    if (m & (1u << 1)) launch_chunk<1>(b, s);
-    if (m & (1u << 2)) launch_chunk<2>(b, s);
-    if (m & (1u << 3)) launch_chunk<3>(b, s);
-    if (m & (1u << 4)) launch_chunk<4>(b, s);
-    if (m & (1u << 5)) launch_chunk<5>(b, s);
-    if (m & (1u << 6)) launch_chunk<6>(b, s);
-    if (m & (1u << 7)) launch_chunk<7>(b, s);
-    if (m & (1u << 8)) launch_chunk<8>(b, s);
-    if (m & (1u << 9)) launch_chunk<9>(b, s);
-    if (m & (1u << 10)) launch_chunk<10>(b, s);
-    if (m & (1u << 11)) launch_chunk<11>(b, s);
-    if (m & (1u << 12)) launch_chunk<12>(b, s);
-    if (m & (1u << 13)) launch_chunk<13>(b, s);
-    if (m & (1u << 14)) launch_chunk<14>(b, s);
-    if (m & (1u << 15)) launch_chunk<15>(b, s);
-    if (m & (1u << 16)) launch_chunk<16>(b, s);
-  }
+  if (b.chunk_p1_mask && b.max_chunks > 0) launch_chunk_fit(b, s);
   if (b.other_cont) {
     if (b.lin_group > 0) launch_linear_tc(b, s);
     k_chi2_other<<<b.E, CT, 0, s>>>(G, b);
@@ -1950,55 +1638,6 @@ __global__ void k_prep_status(EvalBatch b) {
 }
 void launch_prep_status(const EvalBatch &b, cudaStream_t s) {
   k_prep_status<<<(b.E + 255) / 256, 256, 0, s>>>(b);
-  count_launch();
-}
-
-// ChunkFitter::build_continuum_from_chunks (continuum_fitting.rs:228-278)
-// from Legendre coefficients: continuum = blend of the chunk polynomials.
-template <int K>
-__device__ float build_one(const DevStar &st, const double *coef, int i) {
-  const int nc = st.n_chunks;
-  int c = 0;
-  while (c + 1 < nc && i >= st.cstart[c + 1]) c++;
-  float cp[K], cc[K];
-  for (int k = 0; k < K; k++) cc[k] = (float)coef[c * MAX_P1 + k];
-  if (c > 0 && i < st.cstop[c - 1]) {
-    for (int k = 0; k < K; k++) cp[k] = (float)coef[(c - 1) * MAX_P1 + k];
-    const float pv = poly_eval<K>(cp, st.xa[i]);
-    const float cu = poly_eval<K>(cc, st.xb[i]);
-    const float f = st.fac[i];
-    return pv * f + cu * (1.0f - f);
-  }
-  return poly_eval<K>(cc, st.xa[i]);
-}
-
-__global__ void k_build_chunk(const DevStar *stp, const double *coef, int n, float *out) {
-  const DevStar &st = *stp;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    float v;
-    switch (st.p1) {
-      case 1: v = build_one<1>(st, coef, i); break;
-      case 2: v = build_one<2>(st, coef, i); break;
-      case 3: v = build_one<3>(st, coef, i); break;
-      case 4: v = build_one<4>(st, coef, i); break;
-      case 5: v = build_one<5>(st, coef, i); break;
-      case 6: v = build_one<6>(st, coef, i); break;
-      case 7: v = build_one<7>(st, coef, i); break;
-      case 8: v = build_one<8>(st, coef, i); break;
-      case 9: v = build_one<9>(st, coef, i); break;
-      case 10: v = build_one<10>(st, coef, i); break;
-      case 11: v = build_one<11>(st, coef, i); break;
-      case 12: v = build_one<12>(st, coef, i); break;
-      case 13: v = build_one<13>(st, coef, i); break;
-      case 14: v = build_one<14>(st, coef, i); break;
-      case 15: v = build_one<15>(st, coef, i); break;
-      default: v = build_one<16>(st, coef, i); break;
-    }
-    out[i] = v;
-  }
-}
-void launch_build_chunk(const DevStar *star, const double *coef, int n, float *out, cudaStream_t s) {
-  k_build_chunk<<<(n + 255) / 256, 256, 0, s>>>(star, coef, n, out);
   count_launch();
 }
 

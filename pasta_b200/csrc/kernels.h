@@ -144,6 +144,8 @@ void launch_gauss(const DevGrid &G, const EvalBatch &b, cudaStream_t s);
 void launch_resample_obs(const DevGrid &G, const EvalBatch &b, cudaStream_t s);
 // chi2 from the model at the observed pixels (b.given when set)
 void launch_chi2(const DevGrid &G, const EvalBatch &b, cudaStream_t s);
+// chunk continua (chunk.cu), every polynomial order present
+void launch_chunk_fit(const EvalBatch &b, cudaStream_t s);
 // linear-model continua on the tensor cores, every basis width present (lintc.cu)
 void launch_linear_tc(const EvalBatch &b, cudaStream_t s);
 // copy the preparation status to b.status (batches without chi2)
@@ -220,6 +222,7 @@ void launch_pso_update(const DevGrid &G, const Swarm &w, cudaStream_t s);
 // after evaluation: initial sort or best update, iteration counter, done flags
 void launch_pso_best(const Swarm &w, const double *cost, const int *status, cudaStream_t s);
 
+int num_sms();  // of the current device at the first call
 int64_t kernel_launches();
 void count_launch(int n = 1);
 

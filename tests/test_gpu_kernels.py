@@ -1,0 +1,89 @@
+"""Edges of single kernels: tile remainders, the smallest sizes, and the rules
+that choose between two forms of a kernel.  An evaluation's result never
+depends on the batch it is in, so the forms are compared bit for bit; values
+are compared with plain numpy in double precision (chi2 relative 1e-5, the
+tolerance of the other chi2 tests)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+CHI2_TOL = 1e-5
+
+
+@pytest.fixture(scope="module")
+def env():
+    from pasta_b200 import pasta as P
+    from pasta_b200 import synth as S
+    spec = S.config0_grid(n_px=4000)
+    labels, spectra, factors = S.make_grid(spec)
+    wl = P.WlGrid(spec.log_first, spec.log_step, spec.n_px, log=True)
+    interp = P.InMemInterpolator.from_arrays(labels, spectra, factors, wl)
+    star = S.make_star(spec, [7130.0, 0.07, 4.02, 50.0, 20.0], 3001, 100.0, 85000.0, seed=3)
+    return dict(P=P, S=S, spec=spec, interp=interp, wl=wl, star=star)
+
+
+def _near(star, n, seed):
+    rng = np.random.default_rng(seed)
+    lab = star.label + rng.uniform(-1.0, 1.0, (n, 5)) * [300.0, 0.2, 0.2, 30.0, 20.0]
+    return lab
+
+
+def _chunk_chi2(wl, flux, var, model, chunks, degree, overlap=0.2):
+    """chi2 of the blended chunk polynomials of flux / model, in double."""
+    n = len(wl)
+    edge = lambda i: min(max(i / chunks * (wl[-1] - wl[0]) + wl[0], wl[0]), wl[-1])  # noqa: E731
+    start = [0 if c == 0 else int(np.searchsorted(wl, edge(c - overlap), "right")) for c in range(chunks)]
+    stop = [n if c == chunks - 1 else int(np.searchsorted(wl, edge(c + 1 + overlap), "left")) for c in range(chunks)]
+    y, cont, prev = flux / model, np.zeros(n), None
+    for c, (a, b) in enumerate(zip(start, stop)):
+        x = (wl[a:b] - wl[a]) / (wl[b - 1] - wl[a]) * 2.0 - 1.0
+        q, _ = np.linalg.qr(np.polynomial.legendre.legvander(x, degree))
+        fit = np.zeros(n)
+        fit[a:b] = q @ (q.T @ y[a:b])
+        lo = a if c == 0 else stop[c - 1]
+        cont[lo:b] = fit[lo:b]
+        if c:
+            t = (wl[a:lo] - wl[lo - 1]) / (wl[a] - wl[lo - 1])
+            f = np.sin(t * np.pi / 2.0) ** 2
+            cont[a:lo] = prev[a:lo] * f + fit[a:lo] * (1.0 - f)
+        prev = fit
+    r = (flux - cont * model)[50:n - 50]
+    return float((r * r / var[50:n - 50]).sum() / (n - 100))
+
+
+@pytest.mark.parametrize("n,chunks,degree", [(300, 2, 0), (301, 2, 3), (640, 3, 5), (1023, 5, 8), (1025, 4, 7), (2049, 9, 4),
+                                             (4097, 12, 2), (5003, 8, 5), (9001, 17, 9), (3001, 6, 15)])
+@pytest.mark.parametrize("scale", [1.0, 1e-18])
+def test_chunk_fit_edges(env, n, chunks, degree, scale):
+    """Pixel counts around the kernel's blocks of 64, 128 and 256 pixels, fewer and more chunks than warps, and
+    (scale 1e-18) variances around 1e-40, below the normal range, where the fast reciprocal does not hold.  The
+    rounding of such a variance is at most 0.5 * 2^-149 / 4e-41 = 2e-5 of it."""
+    P = env["P"]
+    rng = np.random.default_rng(n)
+    wl = np.geomspace(4100.0, 4900.0, n)
+    model = (0.7 + 0.3 * np.cos(wl / 3.0)).astype(np.float32)
+    sigma = 0.01
+    x = np.linspace(-1.0, 1.0, n)
+    flux = (model * (1.0 + 0.2 * x - 0.1 * x * x) + sigma * rng.standard_normal(n)) * scale
+    flux, var = flux.astype(np.float32), np.full(n, (sigma * scale) ** 2, np.float64)
+    var32 = var.astype(np.float32)
+    got = P.ChunkContinuumFitter(wl, chunks, degree, 0.2).fit_and_return_chi2(model, flux, var32)
+    ref = _chunk_chi2(wl, flux.astype(np.float64), var, model.astype(np.float64), chunks, degree)
+    assert abs(got - ref) <= (CHI2_TOL + (2e-5 if scale < 1.0 else 0.0)) * ref
+
+
+@pytest.mark.parametrize("chunks,degree", [(5, 8), (8, 5), (2, 1), (11, 3)])
+def test_chunk_fit_pairs_match_single_evaluations(env, chunks, degree):
+    """A large batch works pairs of evaluations (an odd number of them here), a small one each alone."""
+    P, star, interp = env["P"], env["star"], env["interp"]
+    disp = P.FixedResolutionDispersion(star.wl, 85000.0, env["wl"])
+    cont = P.ChunkContinuumFitter(star.wl, chunks, degree, 0.2)
+    fitter = interp.get_fitter(disp, cont, P.PSOSettings(8, 2), (0.0, 300.0), (-150.0, 150.0))
+    lab = _near(star, 1301, 5)
+    lab[[3, 10, 11, 1300], 0] = 1e5  # labels outside the grid, alone and as a pair
+    both = np.array(fitter.chi2(interp, star.flux, star.var, lab))
+    assert np.isnan(both[[3, 10, 11, 1300]]).all()
+    for a in (0, 9, 512, 1288):
+        alone = np.array(fitter.chi2(interp, star.flux, star.var, lab[a:a + 13]))
+        np.testing.assert_array_equal(both[a:a + 13], alone)
