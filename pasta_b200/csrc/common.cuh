@@ -105,7 +105,7 @@ struct DevStar {
   double wl_first, wl_last;   // first/last observed wavelength (range check)
   double wl_min, wl_max;      // extreme observed wavelengths (windows on NonUniform grids)
   double fidx_min, fidx_max;  // extreme float indices (windows on uniform grids)
-  const float *gk;      // DISP_FIXED: [gw]; DISP_PIXEL: [npx][gw]
+  const float *gk;      // DISP_FIXED: [gw]; DISP_PIXEL: [gw][npx]
   const float2 *gspec;  // DISP_FIXED: 2048-point spectrum of gk (1025 bins), else null
   const int *cstart, *cstop;  // chunk bounds
   const float *xa, *xb, *fac; // per observed pixel: coordinate in lower/upper chunk, blend factor

@@ -334,7 +334,7 @@ struct pasta_dispersion {
   double wl_first = 0, wl_last = 0, wl_min = 0, wl_max = 0, fidx_min = 0, fidx_max = 0;
   int sorted = 0;  // observed wavelengths and float indices never decrease
   int gw = 0;
-  std::vector<float> gk;  // fixed: [gw]; per pixel: [synth_n][gw]
+  std::vector<float> gk;  // fixed: [gw]; per pixel: [gw][synth_n]
   DBuf<double> dfidx, dwl;
   DBuf<float> dgk;
   DBuf<float2> dgspec;  // fixed kernel: 2048-point spectrum (1025 bins)
@@ -415,8 +415,13 @@ void disp_per_pixel(pasta_dispersion *d, const std::vector<float> &sig) {
   if (w > 2 * 255 + 1) fail(PASTA_E_UNSUPPORTED, "instrument kernel of %d taps exceeds the supported 511", w);
   d->gw = w;
   d->dev_kind = DISP_PIXEL;
-  d->gk.assign((size_t)w * sig.size(), 0.0f);
-  for (size_t i = 0; i < sig.size(); i++) make_gaussian(&d->gk[i * w], w, sig[i]);
+  const size_t n = sig.size();
+  d->gk.resize((size_t)w * n);
+  std::vector<float> k(w);
+  for (size_t i = 0; i < n; i++) {
+    make_gaussian(k.data(), w, sig[i]);
+    for (int t = 0; t < w; t++) d->gk[t * n + i] = k[t];
+  }
 }
 
 }  // namespace
@@ -2023,12 +2028,8 @@ int pasta_dispersion_destroy(pasta_dispersion *d) {
 int pasta_dispersion_kernels(const pasta_dispersion *d, int64_t *width, float *out) {
   return guard([&] {
     *width = d->gw;
-    if (out && d->dev_kind == DISP_PIXEL) {  // width x n_synth row-major
-      for (int64_t i = 0; i < d->synth_n; i++)
-        for (int t = 0; t < d->gw; t++) out[(size_t)t * d->synth_n + i] = d->gk[(size_t)i * d->gw + t];
-    } else if (out && d->dev_kind == DISP_FIXED) {
-      std::copy(d->gk.begin(), d->gk.end(), out);
-    }
+    // per pixel: width x n_synth row-major
+    if (out && (d->dev_kind == DISP_PIXEL || d->dev_kind == DISP_FIXED)) std::copy(d->gk.begin(), d->gk.end(), out);
   });
 }
 

@@ -583,8 +583,12 @@ __device__ __forceinline__ float instrument(const DevStar &st, int N, int i, int
     for (int k = 0; k < w; k++) acc = fmaf(__ldg(&g[k]), r(i + h - k), acc);
   } else {
     if (i < h || i >= N - h) return r(i);
-    const float *kk = st.gk + (size_t)i * w;
-    for (int t = 0; t < w; t++) acc = fmaf(__ldg(&kk[t]), r(i - h + t), acc);
+    // tap-major: the lanes of a warp work neighbouring pixels and read
+    // neighbouring words (pixel-major taps, a stride of w words between the
+    // lanes, made k_broaden 1.51 ms for 1,000 evaluations of 80,000 pixels
+    // and 17 taps; 1.27 ms now)
+    const float *kk = st.gk + i;
+    for (int t = 0; t < w; t++) acc = fmaf(__ldg(&kk[(size_t)t * N]), r(i - h + t), acc);
   }
   return acc;
 }
