@@ -502,97 +502,6 @@ void launch_interp(const DevGrid &G, const EvalBatch &b, cudaStream_t s) {
   }
 }
 
-// ------------------------------------------------------------ resampling
-// shift_and_resample (convolve_rv.rs:569-603): index in double, weight from
-// the f32-rounded index minus the f32 floor, linear interpolation in f32.
-struct ResPos {
-  int j;    // left synth pixel
-  float w;  // weight of pixel j + 1
-};
-__device__ __forceinline__ float resample_value(float w, float sj, float sj1) {
-  return __fadd_rn(__fmul_rn(1.0f - w, sj), __fmul_rn(w, sj1));
-}
-struct Resampler {
-  const float *s;
-  int N, kind;
-  double shift_log, shift_factor, lin_offset;
-  const double *fidx, *wl_obs, *wl_vals;
-  const float *given;  // model given directly at the observed pixels
-  // j never decreases with i when the float indices do not
-  __device__ __forceinline__ ResPos pos(int i) const {
-    double idx;
-    if (kind == WL_LOG) idx = fidx[i] + shift_log;
-    else if (kind == WL_LIN) idx = __dadd_rn(__dmul_rn(shift_factor, fidx[i]), lin_offset);
-    else {
-      const double wl = __dmul_rn(wl_obs[i], shift_factor);
-      bool f;
-      int k = lower_bound(wl_vals, N, wl, f);
-      if (f) idx = (double)k;
-      else if (k == 0) idx = 0.0;
-      else if (k == N) idx = (double)N - 1.0;
-      else idx = __dadd_rn(__dadd_rn(__ddiv_rn(wl - wl_vals[k - 1], wl_vals[k] - wl_vals[k - 1]), (double)k), -1.0);
-    }
-    return from_index(idx);
-  }
-  __device__ __forceinline__ ResPos from_index(double idx) const {
-    const double fl = floor(idx);
-    int j = fl > 0 ? (int)fl : 0;
-    if (j > N - 2) j = N - 2;  // the preparation kernel rejected j + 1 >= N already
-    return ResPos{j, (float)idx - (float)j};
-  }
-  // position from an already loaded float index (uniform grids)
-  __device__ __forceinline__ ResPos pos_from_fidx(double fx) const {
-    return from_index(kind == WL_LOG ? fx + shift_log : __dadd_rn(__dmul_rn(shift_factor, fx), lin_offset));
-  }
-  __device__ __forceinline__ float operator()(int i) const {
-    if (given) return given[i];
-    const ResPos q = pos(i);
-    return resample_value(q.w, s[q.j], s[q.j + 1]);
-  }
-};
-
-__device__ __forceinline__ Resampler make_resampler(const DevGrid &G, const DevStar &st, const EvalPrep &P,
-                                                    const float *row, const float *given) {
-  Resampler r;
-  r.s = row;
-  r.N = G.npx;
-  r.kind = G.wl_kind;
-  r.shift_log = P.shift_log;
-  r.shift_factor = P.shift_factor;
-  r.lin_offset = P.lin_offset;
-  r.fidx = st.fidx;
-  r.wl_obs = st.wl_obs;
-  r.wl_vals = G.wl_vals;
-  r.given = given;
-  return r;
-}
-
-// ------------------------------------------------ instrument profile (tile)
-// FixedTargetDispersionLogSpace: g[i] = sum_k gk[k] r[i + h - k], r zero
-// outside the grid (convolve_rv.rs:207-210).  Per-pixel kernels
-// (VariableTargetDispersion / FixedTargetDispersionNonLog):
-// g[i] = kernel_i . r[i-h .. i+h], pixels within h of either end pass
-// through (convolve_rv.rs:213-233, 414-430).  r(t) reads the rotation
-// output for synth pixel t from wherever the caller staged it.
-template <class RF>
-__device__ __forceinline__ float instrument(const DevStar &st, int N, int i, int h, const RF &r) {
-  const int w = 2 * h + 1;
-  float acc = 0.0f;
-  if (st.disp_kind == DISP_FIXED) {
-    const float *g = st.gk;
-    for (int k = 0; k < w; k++) acc = fmaf(__ldg(&g[k]), r(i + h - k), acc);
-  } else {
-    if (i < h || i >= N - h) return r(i);
-    // tap-major: the lanes of a warp work neighbouring pixels and read
-    // neighbouring words (pixel-major taps, a stride of w words between the
-    // lanes, made k_broaden 1.51 ms for 1,000 evaluations of 80,000 pixels
-    // and 17 taps; 1.27 ms now)
-    const float *kk = st.gk + i;
-    for (int t = 0; t < w; t++) acc = fmaf(__ldg(&kk[(size_t)t * N]), r(i - h + t), acc);
-  }
-  return acc;
-}
-
 // ------------------------------------------------------ fused broadening
 // Asynchronous 16-byte global -> shared copies (cp.async): the next tile's
 // input streams in while the current one is worked.  A copy with ok ==
@@ -604,415 +513,6 @@ __device__ __forceinline__ void cp_async16(float *smem, const float *gmem, bool 
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-struct BroadenItem {
-  int e, pair, m, hg, V, s0, s1, j0, j1;
-  bool has1;
-};
-
-// the work item (evaluation e, block pair), or false when it has nothing to do
-__device__ __forceinline__ bool broaden_item(const EvalBatch &b, int e, int pair, BroadenItem &w) {
-  w.e = e;
-  w.pair = pair;
-  const EvalPrep &P = b.prep[e];
-  if (P.status || !P.fused || 2 * pair >= P.nblk) return false;
-  w.m = P.m;
-  w.hg = P.hg;
-  w.V = FFTN - (w.m - 1) - 2 * w.hg;
-  w.s0 = P.o_lo + 2 * pair * (w.V - 1);
-  w.s1 = w.s0 + (w.V - 1);
-  w.has1 = 2 * pair + 1 < P.nblk;
-  // input t of a block is synth pixel (s - hg - hw + t) for the rotation,
-  // (s - hg + t) for the identity
-  const int shift = w.m > 1 ? w.hg + (w.m - 1) / 2 : w.hg;
-  w.j0 = w.s0 - shift;
-  w.j1 = w.s1 - shift;
-  return true;
-}
-
-// The items of a CTA (item = e * max_pairs + pair) come in runs of ic
-// consecutive items (mostly neighbouring block pairs of one evaluation, so
-// their metadata and the overlap of their inputs are still in cache): run r
-// of the CTA is items [ic R, ic R + ic) with R = blockIdx.x + r gridDim.x.
-struct ItemCursor {
-  int e, pair, k, ic, mp, E;
-  long long run;
-  __device__ __forceinline__ void set_run() {
-    const long long item = run * ic;
-    e = (int)(item / mp);
-    pair = (int)(item % mp);
-    k = 0;
-  }
-  __device__ __forceinline__ void init(const EvalBatch &b, int run_len) {
-    mp = b.max_pairs;
-    E = b.E;
-    ic = run_len;
-    run = blockIdx.x;
-    set_run();
-  }
-  __device__ __forceinline__ void advance() {
-    if (++k < ic) {
-      if (++pair >= mp) {
-        pair = 0;
-        e++;
-      }
-    } else {
-      run += gridDim.x;
-      set_run();
-    }
-  }
-  __device__ __forceinline__ bool done() const { return e >= E; }
-  // move to the first item with work at or after the current one
-  __device__ __forceinline__ void settle(const EvalBatch &b) {
-    BroadenItem w;
-    while (!done() && !broaden_item(b, e, pair, w)) advance();
-  }
-};
-
-// The 2 x 16 inputs of this thread for item w: block input j = 128 n1 + t
-// is synth pixel j0 + j of the interpolated row (zero outside [i_lo, i_hi)).
-// Interior item pairs (both blocks inside the window, the common case) load
-// without per-element bounds tests.
-__device__ __forceinline__ void broaden_inputs(const EvalBatch &b, const BroadenItem &w, const EvalPrep &P,
-                                               float (&x0)[16], float (&x1)[16]) {
-  const float *row = b.bufA + (size_t)w.e * b.stride;
-  const int ilo = P.i_lo, ihi = P.i_hi;
-  if (w.has1 && w.j0 >= ilo && w.j1 + FFTN <= ihi) {
-    const float *r0 = row + w.j0 + (int)threadIdx.x, *r1 = row + w.j1 + (int)threadIdx.x;
-#pragma unroll
-    for (int n1 = 0; n1 < 16; n1++) {
-      x0[n1] = __ldg(r0 + 128 * n1);
-      x1[n1] = __ldg(r1 + 128 * n1);
-    }
-    return;
-  }
-#pragma unroll
-  for (int n1 = 0; n1 < 16; n1++) {
-    const int g0 = w.j0 + 128 * n1 + (int)threadIdx.x, g1 = w.j1 + 128 * n1 + (int)threadIdx.x;
-    x0[n1] = (g0 >= ilo && g0 < ihi) ? __ldg(row + g0) : 0.0f;
-    x1[n1] = (w.has1 && g1 >= ilo && g1 < ihi) ? __ldg(row + g1) : 0.0f;
-  }
-}
-
-constexpr int BT = F2_T;      // threads of k_broaden
-constexpr int BR_RUN = 8;     // longest run of consecutive items a CTA takes
-// dynamic shared memory (bytes): exchange buffers 1 and 2 (buffer 2 also
-// holds the rotation outputs, buffer 1 the outputs of the instrument taps),
-// twiddles of pass 2, the fixed instrument taps
-constexpr int BR_S1 = 0, BR_S2 = BR_S1 + F2_S1 * 8, BR_T2 = BR_S2 + F2_S2 * 8, BR_GK = BR_T2 + 16 * 8 * 8,
-              BR_SMEM = BR_GK + 512 * 4;
-
-// Resampling of an item's observed pixels [q0, q2) (the left synth pixel of
-// [q0, q1) in block 0, of [q1, q2) in block 1) from the final outputs in
-// shared memory, with the wavelength kind fixed at compile time.  The float
-// indices come from the star's table (a star's particles share it; the
-// item prefetched its range into L1 before the transforms); each thread
-// issues the loads of EU pixels before their arithmetic.
-template <int KIND>
-__device__ __forceinline__ void resample_item(const Resampler &R, float *y, const float *ob0,
-                                              const float *ob1, int q0, int q1, int q2, int s0, int s1, int V) {
-  constexpr int EU = 8;
-  for (int i0 = q0 + (int)threadIdx.x; i0 < q2; i0 += EU * BT) {
-    double fx[EU];
-#pragma unroll
-    for (int r = 0; r < EU; r++) {
-      const int i = min(i0 + r * BT, q2 - 1);
-      fx[r] = KIND == WL_NONUNI ? 0.0 : __ldg(&R.fidx[i]);
-    }
-#pragma unroll
-    for (int r = 0; r < EU; r++) {
-      const int i = i0 + r * BT;
-      if (i < q2) {
-        ResPos q;
-        if (KIND == WL_LOG) q = R.from_index(fx[r] + R.shift_log);
-        else if (KIND == WL_LIN) q = R.from_index(__dadd_rn(__dmul_rn(R.shift_factor, fx[r]), R.lin_offset));
-        else q = R.pos(i);
-        const bool k1 = i >= q1;
-        const float *o = k1 ? ob1 : ob0;
-        const int u = min(max(q.j - (k1 ? s1 : s0), 0), V - 2);  // in range by construction of bnd
-        y[i] = resample_value(q.w, o[u], o[u + 1]);
-      }
-    }
-  }
-}
-
-// the pass-1 twiddle W_2048^(t k1) of this thread from W^t, W^2t, W^4t and
-// W^8t (table values, computed in double on the host) by at most three
-// products
-__device__ __forceinline__ cf tw_pass1(int k1, const cf &w1, const cf &w2, const cf &w4, const cf &w8) {
-  cf r = (k1 & 1) ? w1 : cf{1.0f, 0.0f};
-  if (k1 & 2) r = (k1 & 1) ? cmul(r, w2) : w2;
-  if (k1 & 4) r = (k1 & 3) ? cmul(r, w4) : w4;
-  if (k1 & 8) r = (k1 & 7) ? cmul(r, w8) : w8;
-  return r;
-}
-
-// One work item = two overlap-save blocks of one evaluation.  Block k yields
-// V = 2048 - (m - 1) - 2 hg final outputs starting at s_k = o_lo + k (V - 1):
-// the rotation outputs [s - hg, s + V + hg) come from one overlap-save block
-// of 2048 inputs (the reference uses overlap-add, convolve_rv.rs:121-157;
-// both are the same linear convolution), and the instrument profile is then
-// applied from shared memory.  Block k owns synth pixels [s_k, s_k + V - 1);
-// its last output is the partner j + 1 of its last owned pixel j.  The two
-// real blocks ride in the real and imaginary parts of one complex FFT (the
-// kernel is real, so the two products separate after the inverse).  Rotation
-// outputs outside [0, N) are zero, like the reference's cropped segment.
-// With the identity rotation the FFT is skipped.  Away from the grid ends
-// the instrument Gaussian acts on rotation outputs that are all inside
-// [0, N), where rotation-then-Gaussian is one convolution with the combined
-// kernel: the spectra are multiplied (H x G) and the taps are skipped.
-//
-// Epilogue: either the owned synth pixels go to row B, or (chi2 batches,
-// EvalPrep::epi) the block resamples the observed pixels whose left synth
-// pixel it owns (EvalBatch::bnd lists them per block) from shared memory and
-// writes the model at the observed pixels to row B; the synth row never
-// reaches memory.  An item's float indices are prefetched into L1 before its
-// transforms; a CTA takes runs of consecutive items (ItemCursor).
-__global__ void __launch_bounds__(BT, 5) k_broaden(DevGrid G, EvalBatch b, const float2 *__restrict__ tw, int run_len) {
-  extern __shared__ __align__(16) unsigned char br_smem[];
-  float2 *S1 = reinterpret_cast<float2 *>(br_smem + BR_S1);
-  float2 *S2 = reinterpret_cast<float2 *>(br_smem + BR_S2);
-  float2 *T2 = reinterpret_cast<float2 *>(br_smem + BR_T2);
-  float *gks = reinterpret_cast<float *>(br_smem + BR_GK);
-  const int t = threadIdx.x, N = G.npx;
-  // twiddles: T2[k2][n3] = W_128^(n3 k2) in shared memory; W_2048^(t k1)
-  // from the four powers of two of W^t in registers
-  for (int i = t; i < 16 * 8; i += BT) T2[i] = __ldg(&tw[(16 * (i & 7) * (i >> 3)) & (FFTN - 1)]);
-  cf tw1, tw2, tw4, tw8;
-  {
-    const float2 a = __ldg(&tw[t]), c = __ldg(&tw[2 * t]), d = __ldg(&tw[4 * t]), f = __ldg(&tw[8 * t]);
-    tw1 = cf{a.x, a.y};
-    tw2 = cf{c.x, c.y};
-    tw4 = cf{d.x, d.y};
-    tw8 = cf{f.x, f.y};
-  }
-  ItemCursor cur;
-  cur.init(b, run_len);
-  cur.settle(b);
-  const int k1p = t >> 3, n3p = t & 7;  // pass-2 role of this thread
-  int gk_star = -1;                       // star whose instrument taps are in gks
-  while (!cur.done()) {
-    ItemCursor nxt = cur;
-    nxt.advance();
-    nxt.settle(b);
-    BroadenItem w;
-    broaden_item(b, cur.e, cur.pair, w);
-    const int e = w.e, pair = w.pair, m = w.m, hg = w.hg, V = w.V, s0 = w.s0, s1 = w.s1;
-    const bool has1 = w.has1;
-    const EvalPrep &P = b.prep[e];
-    const int nblk = P.nblk, ohi = P.o_hi;
-    const DevStar &st = b.stars[P.star];
-    const bool fixedk = hg > 0 && st.disp_kind == DISP_FIXED;
-    const int gw = 2 * hg + 1;
-    int q0 = 0, q1 = 0, q2 = 0;
-    if (P.epi) {
-      const int *bd = b.bnd + (size_t)e * b.bnd_stride + 2 * pair;
-      q0 = bd[0];
-      q1 = bd[1];
-      q2 = has1 ? bd[2] : q1;
-    }
-    __syncthreads();  // the last item's epilogue is done with the shared buffers
-    // this item's inputs and instrument taps
-    float in0[16], in1[16];
-    broaden_inputs(b, w, P, in0, in1);
-    if (P.epi && G.wl_kind != WL_NONUNI) {  // the float indices the resampling reads: into L1 meanwhile
-      const double *fq = st.fidx + q0;
-      for (int l = t; l * 16 < q2 - q0; l += BT) asm volatile("prefetch.global.L1 [%0];" ::"l"(fq + 16 * l));
-    }
-    const int e_last = min((has1 ? s1 : s0) + V, ohi);
-    const bool fold = fixedk && m > 1 && st.gspec != nullptr && b.HG != nullptr && s0 - hg >= 0 && e_last + hg <= N;
-    if (fixedk && !fold && P.star != gk_star) {  // the taps are applied from shared memory (edge blocks)
-      for (int k = t; k < gw; k += BT) gks[k] = __ldg(&st.gk[k]);
-      gk_star = P.star;
-    }
-    const float sc = 1.0f / 2048.0f;
-    float *ob0, *ob1;  // final outputs u in [0, V) of the two blocks
-    if (m > 1) {
-      cf v[16];
-#pragma unroll
-      for (int n1 = 0; n1 < 16; n1++) v[n1] = cf{in0[n1], in1[n1]};
-      // pass 1: DFT-16 over n1, twiddle, exchange 1
-      dft16<false>(v);
-#pragma unroll
-      for (int k1 = 0; k1 < 16; k1++) {
-        const cf z = k1 ? cmul(v[k1], tw_pass1(k1, tw1, tw2, tw4, tw8)) : v[k1];
-        S1[k1 * F2_XP + t] = make_float2(z.x, z.y);
-      }
-      __syncthreads();
-      // pass 2: DFT-16 over n2, twiddle, exchange 2
-#pragma unroll
-      for (int n2 = 0; n2 < 16; n2++) {
-        const float2 z = S1[k1p * F2_XP + 8 * n2 + n3p];
-        v[n2] = cf{z.x, z.y};
-      }
-      dft16<false>(v);
-#pragma unroll
-      for (int k2 = 0; k2 < 16; k2++) {
-        const cf z = k2 ? cmul_tw<false>(v[k2], T2[k2 * 8 + n3p]) : v[k2];
-        S2[f2_a2(k1p + 16 * k2, n3p)] = make_float2(z.x, z.y);
-      }
-      __syncthreads();
-      // pass 3 (DFT-8 over n3), the spectrum product, and the inverse DFT-8
-      // over k3, for c = t and t + 128; each thread rewrites the slots it read
-      const float2 *H = (fold ? b.HG : b.H) + (size_t)e * 1025;
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int c = t + 128 * h;
-        cf u[8];
-        float2 hk[8];
-        // bins k = c + 256 k3 (c < 256): k < 1024 below k3 = 4, k > 1024
-        // above it (conjugate of bin 2048 - k); k3 = 4 is bin 1024 for c = 0
-#pragma unroll
-        for (int k3 = 0; k3 < 8; k3++) {
-          const int k = c + 256 * k3;
-          if (k3 < 4) {
-            hk[k3] = __ldg(&H[k]);
-          } else if (k3 > 4) {
-            hk[k3] = __ldg(&H[FFTN - k]);
-            hk[k3].y = -hk[k3].y;
-          } else {
-            hk[k3] = __ldg(&H[c == 0 ? 1024 : FFTN - k]);
-            if (c != 0) hk[k3].y = -hk[k3].y;
-          }
-        }
-#pragma unroll
-        for (int n3 = 0; n3 < 8; n3++) {
-          const float2 z = S2[f2_a2(c, n3)];
-          u[n3] = cf{z.x, z.y};
-        }
-        dft8<false>(u);
-#pragma unroll
-        for (int k3 = 0; k3 < 8; k3++) u[k3] = cmul(u[k3], cf{hk[k3].x, hk[k3].y});
-        dft8<true>(u);
-#pragma unroll
-        for (int n3 = 0; n3 < 8; n3++) S2[f2_a2(c, n3)] = make_float2(u[n3].x, u[n3].y);
-      }
-      __syncthreads();
-      // inverse pass 2: conjugate twiddle, DFT-16 over k2, exchange 1
-#pragma unroll
-      for (int k2 = 0; k2 < 16; k2++) {
-        const float2 z = S2[f2_a2(k1p + 16 * k2, n3p)];
-        v[k2] = k2 ? cmul_tw<true>(cf{z.x, z.y}, T2[k2 * 8 + n3p]) : cf{z.x, z.y};
-      }
-      dft16<true>(v);
-#pragma unroll
-      for (int n2 = 0; n2 < 16; n2++) S1[k1p * F2_XP + 8 * n2 + n3p] = make_float2(v[n2].x, v[n2].y);
-      __syncthreads();
-      // inverse pass 1: conjugate twiddle, DFT-16 over k1 -> 2048 x output 128 n1 + t
-#pragma unroll
-      for (int k1 = 0; k1 < 16; k1++) {
-        const float2 z = S1[k1 * F2_XP + t];
-        v[k1] = k1 ? cmul_tw<true>(cf{z.x, z.y}, [&] {
-          const cf q = tw_pass1(k1, tw1, tw2, tw4, tw8);
-          return make_float2(q.x, q.y);
-        }()) : cf{z.x, z.y};
-      }
-      dft16<true>(v);
-      // FFT index i = 128 n1 + t holds rotation output (s - hg) + (i - (m - 1))
-      const int base = m - 1;
-      if (fold) {  // final output u = i - base - 2 hg
-        ob0 = reinterpret_cast<float *>(S2);
-        ob1 = ob0 + 2048;
-#pragma unroll
-        for (int n1 = 0; n1 < 16; n1++) {
-          const int u = 128 * n1 + t - base - 2 * hg;  // at most 2047 - base - 2 hg = V - 1
-          if (u >= 0) {
-            ob0[u] = v[n1].x * sc;
-            ob1[u] = v[n1].y * sc;
-          }
-        }
-      } else {  // rotation outputs r = i - base, zero outside the grid
-        const int r0 = s0 - hg, r1 = s1 - hg;
-#pragma unroll
-        for (int n1 = 0; n1 < 16; n1++) {
-          const int r = 128 * n1 + t - base;
-          if (r >= 0) {
-            const int i0 = r0 + r, i1 = r1 + r;
-            S2[r] = make_float2((i0 >= 0 && i0 < N) ? v[n1].x * sc : 0.0f, (i1 >= 0 && i1 < N) ? v[n1].y * sc : 0.0f);
-          }
-        }
-      }
-    } else {  // identity rotation: the inputs are the rotation outputs r = j
-#pragma unroll
-      for (int n1 = 0; n1 < 16; n1++) S2[128 * n1 + t] = make_float2(in0[n1], in1[n1]);
-    }
-    __syncthreads();
-    if (!fold) {  // instrument taps from the rotation outputs in S2 into buffer 1
-      ob0 = reinterpret_cast<float *>(S1);
-      ob1 = ob0 + 2048;
-      for (int u = t; u < V; u += BT) {
-        const int i0 = s0 + u, i1 = s1 + u;
-        float v0, v1;
-        if (hg == 0) {
-          const float2 x = S2[u];
-          v0 = x.x;
-          v1 = x.y;
-        } else if (fixedk) {  // g[i] = sum_k gk[k] r[i + hg - k]; r[i] sits at i - s + hg
-          float a0 = 0.0f, a1 = 0.0f;
-          for (int k = 0; k < gw; k++) {
-            const float g = gks[k];
-            const float2 x = S2[u + 2 * hg - k];
-            a0 = fmaf(g, x.x, a0);
-            a1 = fmaf(g, x.y, a1);
-          }
-          v0 = a0;
-          v1 = a1;
-        } else {
-          v0 = instrument(st, N, i0, hg, [&](int i) { return S2[i - (s0 - hg)].x; });
-          v1 = has1 ? instrument(st, N, i1, hg, [&](int i) { return S2[i - (s1 - hg)].y; }) : 0.0f;
-        }
-        ob0[u] = v0;
-        ob1[u] = v1;
-      }
-      __syncthreads();
-    }
-    float *y = b.bufB + (size_t)e * b.stride;
-    if (P.epi) {
-      // observed pixels [q0, q2) have their left synth pixel in this item's
-      // blocks; the boundary between them is q1
-      const Resampler R = make_resampler(G, st, P, nullptr, nullptr);
-      if (R.kind == WL_LOG) resample_item<WL_LOG>(R, y, ob0, ob1, q0, q1, q2, s0, s1, V);
-      else if (R.kind == WL_LIN) resample_item<WL_LIN>(R, y, ob0, ob1, q0, q1, q2, s0, s1, V);
-      else resample_item<WL_NONUNI>(R, y, ob0, ob1, q0, q1, q2, s0, s1, V);
-    } else {
-      // owned pixels; the last block also writes its final output
-      const int n0 = 2 * pair + 1 == nblk ? V : V - 1, n1 = 2 * pair + 2 == nblk ? V : V - 1;
-      for (int u = t; u < V; u += BT) {
-        const int i0 = s0 + u, i1 = s1 + u;
-        if (u < n0 && i0 < ohi) y[i0] = ob0[u];
-        if (has1 && u < n1 && i1 < ohi) y[i1] = ob1[u];
-      }
-    }
-    cur = nxt;
-  }
-}
-
-void launch_broaden(const DevGrid &G, const EvalBatch &b, const float2 *tw, cudaStream_t s) {
-  if (b.E <= 0 || b.max_pairs <= 0) return;
-  const size_t smem = BR_SMEM;
-  static int per_sm[64] = {};  // resident CTAs per SM, per device
-  int dev = 0;
-  cudaGetDevice(&dev);
-  int fit = 5;
-  if (dev >= 0 && dev < 64) {
-    if (!per_sm[dev]) {
-      cudaFuncSetAttribute(k_broaden, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      int n = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_broaden, BT, smem) != cudaSuccess || n < 1) n = 1;
-      per_sm[dev] = n;
-    }
-    fit = per_sm[dev];
-  }
-  const long long total = (long long)b.E * b.max_pairs;
-  long long grid = (long long)num_sms() * fit;  // persistent: the CTAs that fit at once
-  if (grid > total) grid = total;
-  // runs of up to BR_RUN consecutive items, as long as every CTA still gets
-  // 16 runs or more (small batches keep single items spread over all CTAs)
-  int run_len = (int)std::min<long long>(BR_RUN, std::max<long long>(1, total / (grid * 16)));
-  if (const char *rl = getenv("PASTA_BR_RUN")) run_len = std::max(1, atoi(rl));
-  k_broaden<<<(unsigned)grid, BT, smem, s>>>(G, b, tw, run_len);
-  count_launch();
-}
 
 // ----------------------------------------------- direct broadening (narrow)
 // Evaluations whose combined kernel (m rotation taps + 2 hg instrument taps)

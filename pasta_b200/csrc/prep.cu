@@ -147,7 +147,8 @@ __global__ void k_prep(DevGrid G, EvalBatch b, int full_window) {
 
 // One CTA per evaluation: the limb-darkened rotation profile
 // (convolve_rv.rs:438-475), normalised by its f32 sum, zero padded to 2048
-// and transformed; the 1025-bin half spectrum goes to H.
+// and transformed; the 1025-bin half spectrum goes to H (times 1/2048 for
+// k_broaden).
 __global__ void __launch_bounds__(FFT_T) k_rotker(DevGrid G, EvalBatch b, const float2 *__restrict__ tw) {
   __shared__ float2 c[FFT_SM];
   __shared__ float red[FFT_T];
@@ -188,7 +189,13 @@ __global__ void __launch_bounds__(FFT_T) k_rotker(DevGrid G, EvalBatch b, const 
   }
   fft2048<false>(c, tw);
   float2 *H = b.H + (size_t)e * 1025;
-  for (int k = threadIdx.x; k <= 1024; k += FFT_T) H[k] = c[pidx(k)];
+  // k_broaden's round trip needs 1/2048, a power of two: scaling its spectra
+  // instead of its outputs changes no bit of them
+  const float sc = P.fused ? 1.0f / 2048.0f : 1.0f;
+  for (int k = threadIdx.x; k <= 1024; k += FFT_T) {
+    const float2 x = c[pidx(k)];
+    H[k] = make_float2(x.x * sc, x.y * sc);
+  }
   // rotation x instrument spectrum for the blocks of the broadening kernel
   // that apply both as one convolution
   const DevStar &st = b.stars[P.star];
@@ -198,7 +205,7 @@ __global__ void __launch_bounds__(FFT_T) k_rotker(DevGrid G, EvalBatch b, const 
       const float2 g = st.gspec[k];
       const float2 x = c[pidx(k)];
       const cf z = cmul(cf{x.x, x.y}, cf{g.x, g.y});
-      HG[k] = make_float2(z.x, z.y);
+      HG[k] = make_float2(z.x * sc, z.y * sc);
     }
   }
 }

@@ -87,3 +87,35 @@ def test_chunk_fit_pairs_match_single_evaluations(env, chunks, degree):
     for a in (0, 9, 512, 1288):
         alone = np.array(fitter.chi2(interp, star.flux, star.var, lab[a:a + 13]))
         np.testing.assert_array_equal(both[a:a + 13], alone)
+
+
+@pytest.mark.parametrize("n_obs", [1, 37, 129, 1024, 1025, 3800])
+@pytest.mark.parametrize("vsini,rv", [(20.0, 0.0), (150.0, -0.0), (299.0, 0.0), (60.0, -40.0)])
+def test_resampling_of_broadening_blocks(env, n_obs, vsini, rv):
+    """The resampling inside the broadening kernel: observed pixels from the very first grid pixel (float index 0) on,
+    fewer than a round of the kernel's threads, exact rounds, one more; against the oracle in double."""
+    import oracle as O
+    P, S, spec, interp = env["P"], env["S"], env["spec"], env["interp"]
+    wl_grid = spec.wl()
+    first = wl_grid[0] if rv == 0.0 else wl_grid[0] * 1.01
+    wl = np.geomspace(first, wl_grid[3800], n_obs)
+    wl[0] = first
+    labels, spectra, factors = S.make_grid(spec)
+    og = O.Grid(labels, spectra, factors, O.WL_LOGSPACE, spec.log_first, spec.log_step)
+    rng = np.random.default_rng(n_obs)
+    flux = (1.0 + 0.1 * rng.standard_normal(n_obs)).astype(np.float32)
+    var = np.full(n_obs, 0.01, np.float32)
+    ones = np.ones(n_obs, np.float32)
+    lab = np.array([[7130.0, 0.07, 4.02, vsini, rv]])
+    disp, cont = P.FixedResolutionDispersion(wl, 85000.0, env["wl"]), P.FixedContinuum(ones)
+    fitter = interp.get_fitter(disp, cont, P.PSOSettings(8, 2), (0.0, 300.0), (-150.0, 150.0))
+    keep = interp.direct_max
+    try:
+        interp.direct_max = 0  # the FFT path
+        got = fitter.chi2(interp, flux, var, lab)[0]
+    finally:
+        interp.direct_max = keep
+    od, oc = O.Disp(og, O.DISP_FIXED, wl, 85000.0), O.Cont(O.CONT_FIXED, continuum=ones)
+    ref, st = O.chi2(og, od, oc, flux, var, lab, O.F64)
+    assert st[0] == 0
+    assert abs(got - ref[0]) <= CHI2_TOL * ref[0]
