@@ -1738,7 +1738,9 @@ void tune_interp_tc(pasta_grid *g) {
     if (getenv("PASTA_TUNE_VERBOSE"))
       fprintf(stderr, "pasta_b200 tune: %lld px, groups of %d: CUDA cores %.4f ms, tensor cores %.4f ms\n",
               (long long)g->npx, gs, tm[0], tm[1]);
-    if (tm[1] < tm[0]) {
+    // a near-tie stays with the CUDA cores: the two forms round differently,
+    // and the choice should not vary from one process to the next
+    if (tm[1] < 0.95f * tm[0]) {
       if (best > SEG) best = gs;
     } else {
       best = SEG + 1;  // the tensor cores must win from the threshold on

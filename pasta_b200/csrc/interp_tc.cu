@@ -61,7 +61,7 @@ constexpr int NA = 2;              // A ring
 constexpr int ND = 4;              // accumulators in tensor memory
 constexpr int DCOLS = 64;          // columns of an accumulator (members)
 constexpr int TMEM_COLS = ND * DCOLS;
-constexpr int TSLAB = 64;          // tiles per item
+constexpr int TSLAB = 64;          // tiles per item at most
 constexpr int S_TC_TIMEOUT = -99;  // PASTA_E_INTERNAL
 
 // warp roles
@@ -198,8 +198,21 @@ __device__ __forceinline__ uint32_t bf16_bits(float x) {
 }
 __device__ __forceinline__ float bf16_val(uint32_t bits) { return __uint_as_float(bits << 16); }
 
-// An item: tiles of one tensor-core group over one slab of TSLAB tiles.
-// Every role derives the same items, in the same order, from the group list.
+// Tiles per item: TSLAB, halved (down to 2) until there are 4 items or more
+// for every CTA, so that few groups still spread over the GPU and the last
+// round of items is short.  An item costs its weights (written by the
+// converters while the last tiles of the item before multiply), so two tiles
+// at least.  One group of 40 members over 20,000 pixels: 102 us with 64 tiles
+// an item (3 CTAs at work), 15 us now.  Every pixel is computed the same way in
+// any item.
+__device__ __forceinline__ int tc_slab(int ngroups, int npx) {
+  const int tiles = (npx + TPX - 1) / TPX;
+  int ts = TSLAB;
+  while (ts > 2 && (long long)ngroups * ((tiles + ts - 1) / ts) < 4ll * gridDim.x) ts >>= 1;
+  return ts;
+}
+// An item: tiles of one tensor-core group over one slab of tiles.  Every
+// role derives the same items, in the same order, from the group list.
 struct TcItem {
   const TcGroup *R;
   int nm, NP;       // members, MMA N (members rounded up to 16)
@@ -207,13 +220,13 @@ struct TcItem {
   int tc_hi;        // tiles cover [lo, tc_hi); [max(lo, tail_start), hi) is the tail
   int ntiles;
 };
-__device__ __forceinline__ bool tc_item(const DevGrid &G, const EvalBatch &b, int item, int slabs, TcItem &I) {
+__device__ __forceinline__ bool tc_item(const DevGrid &G, const EvalBatch &b, int item, int slabs, int ts, TcItem &I) {
   I.R = &b.tcrec[b.tclist[item / slabs]];
   I.nm = I.R->nmem;
   I.NP = (I.nm + 15) & ~15;
-  const int slab0 = (item % slabs) * TSLAB * TPX;
+  const int slab0 = (item % slabs) * ts * TPX;
   I.lo = max(I.R->lo & ~(TPX - 1), slab0);
-  I.hi = min(I.R->hi, slab0 + TSLAB * TPX);
+  I.hi = min(I.R->hi, slab0 + ts * TPX);
   I.tc_hi = min(I.hi, G.tail_start);
   I.ntiles = I.tc_hi > I.lo ? (I.tc_hi - I.lo + TPX - 1) / TPX : 0;
   return I.lo < I.hi;
@@ -221,8 +234,8 @@ __device__ __forceinline__ bool tc_item(const DevGrid &G, const EvalBatch &b, in
 
 }  // namespace
 
-// Persistent CTAs over the items (tensor-core group, slab of TSLAB tiles)
-// of the groups k_group listed, item = blockIdx.x, blockIdx.x + gridDim.x,
+// Persistent CTAs over the items (tensor-core group, slab of tiles) of the
+// groups k_group listed, item = blockIdx.x, blockIdx.x + gridDim.x,
 // ...; tensor memory is allocated once per CTA and every ring's phases run
 // on across items.  Ring slot of the g-th use (g counted over the CTA's
 // tiles): g % size; its full barrier completes for the (g / size)-th time
@@ -231,8 +244,9 @@ __device__ __forceinline__ bool tc_item(const DevGrid &G, const EvalBatch &b, in
 __global__ void __launch_bounds__(TT, 1) k_interp_tc(DevGrid G, EvalBatch b, const __grid_constant__ CUtensorMap tmap) {
   extern __shared__ __align__(1024) unsigned char sm[];
   const int t = threadIdx.x, w = t >> 5, lane = t & 31;
-  const int slabs = (G.npx + TSLAB * TPX - 1) / (TSLAB * TPX);
-  const int nitems = *b.tclist_count * slabs;
+  const int ngroups = *b.tclist_count, ts = tc_slab(ngroups, G.npx);
+  const int slabs = (G.npx + ts * TPX - 1) / (ts * TPX);
+  const int nitems = ngroups * slabs;
   if ((int)blockIdx.x >= nitems) return;
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
   auto bar = [&](int i) { return sbase + SB_BAR + 8u * (uint32_t)i; };
@@ -276,7 +290,7 @@ __global__ void __launch_bounds__(TT, 1) k_interp_tc(DevGrid G, EvalBatch b, con
     bool stop = false;
     for (int item = blockIdx.x; item < nitems && !stop; item += gridDim.x) {
       TcItem I;
-      if (!tc_item(G, b, item, slabs, I)) continue;
+      if (!tc_item(G, b, item, slabs, ts, I)) continue;
       // the rows of this group (a missing row has weight 0: row 0 stands in);
       // lane l < 16 gathers rows 4l .. 4l + 3
       const int k0 = 4 * (lane & 15);
@@ -309,7 +323,7 @@ __global__ void __launch_bounds__(TT, 1) k_interp_tc(DevGrid G, EvalBatch b, con
       long long it = 0;  // items
       for (int item = blockIdx.x; item < nitems && !*err; item += gridDim.x) {
         TcItem I;
-        if (!tc_item(G, b, item, slabs, I)) continue;
+        if (!tc_item(G, b, item, slabs, ts, I)) continue;
         const int bb = (int)(it & 1);
         if (!mbar_wait(bar(B_BFULL + bb), (uint32_t)((it >> 1) & 1))) *err = 1;
         tc_fence_after();
@@ -349,7 +363,7 @@ __global__ void __launch_bounds__(TT, 1) k_interp_tc(DevGrid G, EvalBatch b, con
     bool stop = false;
     for (int item = blockIdx.x; item < nitems && !stop; item += gridDim.x) {
       TcItem I;
-      if (!tc_item(G, b, item, slabs, I)) continue;
+      if (!tc_item(G, b, item, slabs, ts, I)) continue;
       // this item's weights: B_j[n][k] = part j of weight_n,k x factor_k
       const int bb = (int)(it & 1);
       stop = it >= 2 ? !warp_wait(bar(B_BEMPTY + bb), (uint32_t)(((it >> 1) - 1) & 1), err) : warp_stop(err);
@@ -427,7 +441,7 @@ __global__ void __launch_bounds__(TT, 1) k_interp_tc(DevGrid G, EvalBatch b, con
     bool stop = false;  // uniform within a warp; made uniform over the epilogue warps at each item
     for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
       TcItem I;
-      if (!tc_item(G, b, item, slabs, I)) continue;
+      if (!tc_item(G, b, item, slabs, ts, I)) continue;
       // the previous item's table is no longer read; stop together
       if (ep_any(stop || *err != 0)) break;
       if (e < 64) {
