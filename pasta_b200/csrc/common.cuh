@@ -6,6 +6,7 @@
 // src/cubic.rs, src/bounds.rs, src/particleswarm.rs) in code that runs both
 // on the host (set-up, the plain path) and inside the kernels.
 #pragma once
+#include <stddef.h>
 #include <stdint.h>
 
 #include <cmath>
@@ -24,6 +25,7 @@ constexpr int MAX_CHUNKS = 32;
 constexpr int MAX_P1 = 16;          // polynomial order + 1
 constexpr int MAX_LIN_K = 128;      // linear-model columns
 constexpr int MAX_PARTICLES = 1024;
+constexpr int AXIS_KEY = 1 << 14;    // axis points an EvalPrep::key distinguishes
 // the fused broadening kernel needs this many outputs per 2048-point block
 constexpr int MIN_FUSED_OUTPUTS = 128;
 // direct (non-FFT) broadening: outputs per tile, and the widest combined
@@ -117,7 +119,7 @@ struct DevStar {
 };
 
 // Per-evaluation record written by the preparation kernel.
-struct EvalPrep {
+struct alignas(16) EvalPrep {
   int status;
   int star;
   int m;          // rotation kernel width (odd); 1 = identity
@@ -136,9 +138,15 @@ struct EvalPrep {
   double shift_factor; // 1 - rv/c
   double lin_offset;   // Linspace: (start / step) * (shift_factor - 1)
   double vsini;
+  // the neighbour columns as one number (present (teff, logg) pairs and [M/H]
+  // neighbours, and the index of the second neighbour on each axis): equal
+  // exactly when cols are, up to AXIS_KEY points per axis
+  unsigned long long key;
   int cols[64];
   float w[64];
 };
+
+static_assert(offsetof(EvalPrep, cols) % 16 == 0, "k_prep writes cols and w as 16-byte vectors");
 
 struct PsoParams {
   int P;

@@ -6,6 +6,35 @@
 
 namespace pb {
 
+// The grid's axes and limits copied into shared memory by the CTA (the
+// searches and limit scans of the label checks walk them with dependent
+// reads), or the resident ones when they do not fit.  Holds a CTA barrier.
+constexpr int GEOM_SMEM = 8192;
+__device__ __forceinline__ GridGeom geom_shared(const GridGeom &g, double *buf) {
+  const int nt = g.nt, nm = g.nm, nl = g.nl;
+  if ((3 * nt + nm + nl) * 8 > GEOM_SMEM) return g;
+  double *tv = buf, *mv = tv + nt, *lv = mv + nm;
+  int64_t *cum = reinterpret_cast<int64_t *>(lv + nl);
+  int *llo = reinterpret_cast<int *>(cum + nt), *lhi = llo + nt;
+  for (int i = threadIdx.x; i < nt; i += blockDim.x) {
+    tv[i] = g.tv[i];
+    cum[i] = g.cum[i];
+    llo[i] = g.llo[i];
+    lhi[i] = g.lhi[i];
+  }
+  for (int i = threadIdx.x; i < nm; i += blockDim.x) mv[i] = g.mv[i];
+  for (int i = threadIdx.x; i < nl; i += blockDim.x) lv[i] = g.lv[i];
+  __syncthreads();
+  GridGeom r = g;
+  r.tv = tv;
+  r.mv = mv;
+  r.lv = lv;
+  r.cum = cum;
+  r.llo = llo;
+  r.lhi = lhi;
+  return r;
+}
+
 // Bulk prefetch of floats [lo, hi) of a row into L2 (one instruction, issued
 // by one thread; a hint, nothing waits for it).  The row must start on a
 // 16-byte boundary and hold hi rounded up to 4 floats.

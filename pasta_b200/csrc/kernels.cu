@@ -50,10 +50,14 @@ int num_sms() {
 // reference order (rows another member needs add exactly 0), so the result
 // is the same as interpolating every evaluation alone.
 
-__device__ __forceinline__ unsigned long long cols_hash(const int *c) {
-  unsigned long long h = 1469598103934665603ull;  // FNV-1a over the 64 indices
-  for (int n = 0; n < 64; n++) h = (h ^ (unsigned)c[n]) * 1099511628211ull;
-  return h;
+// whether evaluations e and u have the same neighbour columns (keys a, c)
+__device__ __forceinline__ bool same_cols(const DevGrid &G, const EvalBatch &b, int e, unsigned long long a, int u,
+                                          unsigned long long c) {
+  if (a != c) return false;
+  if (max(G.g.nt, max(G.g.nm, G.g.nl)) <= AXIS_KEY) return true;
+  for (int n = 0; n < 64; n++)
+    if (b.prep[e].cols[n] != b.prep[u].cols[n]) return false;
+  return true;
 }
 
 // Segment s of a batch: [start, start + len), a chunk of at most SEG
@@ -71,268 +75,208 @@ int num_segments(const EvalBatch &b) {
   return (b.E + L - 1) / L * ((L + SEG - 1) / SEG);
 }
 
-// One CTA per segment: slice 0 (SEG threads) finds the groups, then
-// GROUP_SLICES slices of SEG threads write the group records, one group per
-// slice at a time (thread t of a slice handles neighbour row t).  Columns
-// shared by TC_MIN_MEMBERS or more evaluations form tensor-core groups
-// (with the tensor-core path on); the others form groups of up to GROUP_MAX.
-constexpr int GROUP_SLICES = 4;
-__global__ void __launch_bounds__(SEG *GROUP_SLICES) k_group(DevGrid G, EvalBatch b) {
-  __shared__ unsigned long long hs[SEG];
-  __shared__ int ok[SEG], lead[SEG], gid[SEG], slot[SEG], open_g[SEG], fill[SEG], cnt_l[SEG], tcg[SEG];
-  __shared__ int ng, ntc;
-  __shared__ int cnt[GROUP_SLICES][2];
-  __shared__ int mem[GROUP_SLICES][GROUP_MAX];
-  const int s = blockIdx.x, tid = threadIdx.x, t = tid % SEG, sl = tid / SEG;
+// The record of a group by one warp: the rows any member (evaluations
+// mem[0 .. GROUP_MAX), -1: unused) weighs, in reference order, with every
+// member's weight, padded to a multiple of 8 rows with zero weights.
+__device__ __forceinline__ void write_group(const DevGrid &G, const EvalBatch &b, GroupRec &R, const int *mem, int lane) {
+  int c[2], nm = 0;
+  float f[2], w[2][GROUP_MAX], wf[2][GROUP_MAX];
+  unsigned bal[2];
+#pragma unroll
+  for (int m = 0; m < GROUP_MAX; m++) nm += mem[m] >= 0;
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int i = lane + 32 * h;
+    c[h] = b.prep[mem[0]].cols[i];
+    f[h] = c[h] >= 0 ? G.factor[c[h]] : 0.0f;
+    bool keep = false;
+#pragma unroll
+    for (int m = 0; m < GROUP_MAX; m++) {
+      w[h][m] = (m < nm && c[h] >= 0) ? b.prep[mem[m]].w[i] : 0.0f;
+      wf[h][m] = w[h][m] * f[h];
+      keep |= wf[h][m] != 0.0f;
+    }
+    bal[h] = __ballot_sync(0xffffffffu, keep);
+  }
+  const unsigned below = (1u << lane) - 1u;
+  const int kept = __popc(bal[0]) + __popc(bal[1]), padded = (kept + 7) & ~7;
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int pos = (h ? __popc(bal[0]) : 0) + __popc(bal[h] & below);
+    if (bal[h] >> lane & 1u) {
+      R.wf[pos][0] = make_float4(wf[h][0], wf[h][1], wf[h][2], wf[h][3]);
+      R.wf[pos][1] = make_float4(wf[h][4], wf[h][5], wf[h][6], wf[h][7]);
+      R.w[pos][0] = make_float4(w[h][0], w[h][1], w[h][2], w[h][3]);
+      R.w[pos][1] = make_float4(w[h][4], w[h][5], w[h][6], w[h][7]);
+      R.col[pos] = c[h];
+      R.f[pos] = f[h];
+    }
+  }
+  if (lane < padded - kept) {  // zero-weight padding rows (add exactly 0)
+    const float4 z4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const int pos = kept + lane;
+    R.wf[pos][0] = R.wf[pos][1] = R.w[pos][0] = R.w[pos][1] = z4;
+    R.col[pos] = 0;
+    R.f[pos] = 0.0f;
+  }
+  if (lane < GROUP_MAX) R.member[lane] = mem[lane];
+  if (lane == 0) {
+    R.nmem = nm;
+    R.nn = padded;
+  }
+}
+
+// One CTA per segment: SEG threads find the groups, then every warp writes
+// group records (a lane per neighbour row and its 32nd next).  Columns shared
+// by TC_MIN_MEMBERS or more evaluations form tensor-core groups (with the
+// tensor-core path on); the others form groups of up to GROUP_MAX, numbered
+// in evaluation order.  All of it is latency: with the columns compared one
+// by one, the groups numbered by one thread and 4 records written at a time
+// between CTA barriers a segment took 41-60 us, 15-22 us now (cold, under ncu).
+constexpr int GROUP_T = 512, GROUP_W = GROUP_T / 32;
+__global__ void __launch_bounds__(GROUP_T) k_group(DevGrid G, EvalBatch b) {
+  __shared__ unsigned long long key[SEG];
+  __shared__ int ok[SEG], lead[SEG], cnt[SEG], tcg[SEG], tclead[TC_MAX_GROUPS];
+  __shared__ int opened[SEG][SEG / GROUP_MAX], mem[SEG][GROUP_MAX];
+  __shared__ unsigned bal[2][2];
+  const int s = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
   int start, len;
   seg_range(b, s, start, len);
   if (len <= 0) {
-    if (tid == 0) {
+    if (t == 0) {
       b.gcount[s] = 0;
       if (b.tccount) b.tccount[s] = 0;
     }
     return;
   }
   const int e = start + t;
-  if (sl == 0) {
-    const bool v = t < len && b.prep[e].status == 0;
-    ok[t] = v;
-    hs[t] = v ? cols_hash(b.prep[e].cols) : 0ull;
-    cnt_l[t] = 0;
-    tcg[t] = -1;
+  int L = -1, rank = 0, n = 0;
+  if (t < SEG) {
+    ok[t] = t < len && b.prep[e].status == 0;
+    key[t] = ok[t] ? b.prep[e].key : 0ull;
   }
+  for (int i = t; i < SEG * GROUP_MAX; i += GROUP_T) mem[i / GROUP_MAX][i % GROUP_MAX] = -1;
   __syncthreads();
-  if (sl == 0) {  // leader: the first earlier evaluation with the same columns
-    int L = ok[t] ? t : -1;
-    if (ok[t]) {
-      const int *c = b.prep[e].cols;
-      for (int u = 0; u < t; u++) {
-        if (!ok[u] || hs[u] != hs[t]) continue;
-        const int *cu = b.prep[start + u].cols;
-        bool same = true;
-        for (int n = 0; n < 64 && same; n++) same = cu[n] == c[n];
-        if (same) {
-          L = u;
-          break;
+  if (t < SEG) {  // leader: the first evaluation with the same columns; rank among them, their number
+    if (ok[t])
+      for (int u = 0; u < SEG; u++)
+        if (ok[u] && same_cols(G, b, e, key[t], start + u, key[u])) {
+          if (L < 0) L = u;
+          rank += u < t;
+          n++;
         }
-      }
-      atomicAdd(&cnt_l[L], 1);
-    }
     lead[t] = L;
-    open_g[t] = -1;
-    fill[t] = 0;
+    cnt[t] = n;
+    const bool tc = L == t && b.tcrec && n >= max(b.tc_min, TC_MIN_MEMBERS);
+    const unsigned m = __ballot_sync(0xffffffffu, tc);
+    if (lane == 0) bal[0][warp] = m;
+    tcg[t] = tc ? __popc(m & ((1u << lane) - 1u)) : -1;  // within the warp
   }
   __syncthreads();
-  if (tid == 0) {
-    // tensor-core groups, in leader order
-    int nt = 0;
-    if (b.tcrec)
-      for (int u = 0; u < SEG; u++)
-        if (ok[u] && lead[u] == u && cnt_l[u] >= max(b.tc_min, TC_MIN_MEMBERS) && nt < TC_MAX_GROUPS) tcg[u] = nt++;
-    ntc = nt;
-    if (b.tccount) b.tccount[s] = nt;
-    if (nt > 0) {
-      const int at = atomicAdd(b.tclist_count, nt);
-      for (int k = 0; k < nt; k++) b.tclist[at + k] = start + k;
-    }
-    // the other evaluations in groups of at most GROUP_MAX, in evaluation order
-    int n = 0;
-    for (int u = 0; u < SEG; u++) {
-      gid[u] = -1;
-      if (!ok[u] || tcg[lead[u]] >= 0) continue;
-      const int l = lead[u];
-      if (open_g[l] < 0 || fill[l] == GROUP_MAX) {
-        open_g[l] = n++;
-        fill[l] = 0;
+  if (t < SEG && warp == 1 && tcg[t] >= 0) tcg[t] += __popc(bal[0][0]);
+  if (t < SEG && tcg[t] >= 0) tclead[tcg[t]] = t;  // at most SEG / TC_MIN_MEMBERS groups
+  const int ntc = __popc(bal[0][0]) + __popc(bal[0][1]);
+  __syncthreads();
+  bool open = false;
+  if (t < SEG) {  // a group opens at every GROUP_MAX-th evaluation of a leader
+    open = ok[t] && tcg[L] < 0 && rank % GROUP_MAX == 0;
+    const unsigned m = __ballot_sync(0xffffffffu, open);
+    if (lane == 0) bal[1][warp] = m;
+    if (open) opened[L][rank / GROUP_MAX] = __popc(m & ((1u << lane) - 1u));
+  }
+  __syncthreads();
+  const int ng = __popc(bal[1][0]) + __popc(bal[1][1]);
+  if (open && warp == 1) opened[L][rank / GROUP_MAX] += __popc(bal[1][0]);
+  __syncthreads();
+  if (t < SEG && ok[t] && tcg[L] < 0) {
+    const int g = opened[L][rank / GROUP_MAX];
+    mem[g][rank % GROUP_MAX] = e;
+    if (b.mkey && n == 1) {  // alone in its segment: offer it to the batch-wide table of column sets
+      const unsigned long long k = key[t];
+      unsigned slot = (unsigned)((k * 0x9E3779B97F4A7C15ull) >> 32) & (unsigned)(b.mtab - 1);
+      for (int probe = 0; probe < b.mtab; probe++) {  // the table is at most half full
+        const unsigned long long old = atomicCAS(&b.mkey[slot], 0ull, k);
+        if (old == 0ull || old == k) break;
+        slot = (slot + 1) & (unsigned)(b.mtab - 1);
       }
-      gid[u] = open_g[l];
-      slot[u] = fill[l]++;
+      const int r = atomicAdd(&b.mcnt[slot], 1);
+      if (r < MERGE_CAP) b.mmem[(size_t)slot * MERGE_CAP + r] = e;
+      if (r == 1) b.mslot[1 + atomicAdd(&b.mslot[0], 1)] = (int)slot;
+      b.erec[e] = start + g;
     }
-    ng = n;
-    b.gcount[s] = n;
+  }
+  if (t == 0) {
+    b.gcount[s] = ng;
+    if (b.tccount) b.tccount[s] = ntc;
+    if (ntc > 0) {
+      const int at = atomicAdd(b.tclist_count, ntc);
+      for (int k = 0; k < ntc; k++) b.tclist[at + k] = start + k;
+    }
   }
   __syncthreads();
-  if (sl == 0 && b.mkey && ok[t] && tcg[lead[t]] < 0 && cnt_l[lead[t]] == 1) {
-    // alone in its segment: offer it to the batch-wide table of column sets
-    const unsigned long long key = hs[t] | 1ull;
-    unsigned slot = (unsigned)(key ^ (key >> 31)) & (unsigned)(b.mtab - 1);
-    for (int probe = 0; probe < b.mtab; probe++) {  // the table is at most half full
-      const unsigned long long old = atomicCAS(&b.mkey[slot], 0ull, key);
-      if (old == 0ull || old == key) break;
-      slot = (slot + 1) & (unsigned)(b.mtab - 1);
+  // tensor-core group records, a warp per group
+  for (int g = warp; g < ntc; g += GROUP_W) {
+    TcGroup &T = b.tcrec[start + g];
+    const int l = tclead[g];
+    int lo = 1 << 30, hi = 0;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int i = lane + 32 * h, c = b.prep[start + l].cols[i];
+      T.col[i] = c;
+      T.f[i] = c >= 0 ? G.factor[c] : 0.0f;
+      if (ok[i] && lead[i] == l) {
+        lo = min(lo, b.prep[start + i].i_lo);
+        hi = max(hi, b.prep[start + i].i_hi);
+      }
     }
-    const int r = atomicAdd(&b.mcnt[slot], 1);
-    if (r < MERGE_CAP) b.mmem[(size_t)slot * MERGE_CAP + r] = e;
-    if (r == 1) b.mslot[1 + atomicAdd(&b.mslot[0], 1)] = (int)slot;
-    b.erec[e] = start + gid[t];
-  }
-  // tensor-core group records: slice sl writes groups sl, sl + GROUP_SLICES,
-  // ... (thread t: row t, member t)
-  for (int tg = sl; tg < ntc; tg += GROUP_SLICES) {
-    int l = -1;
-    for (int u = 0; u < SEG; u++)
-      if (ok[u] && lead[u] == u && tcg[u] == tg) l = u;
-    TcGroup &T = b.tcrec[start + tg];
-    const int c = b.prep[start + l].cols[t];
-    T.col[t] = c;
-    T.f[t] = c >= 0 ? G.factor[c] : 0.0f;
-    // members in evaluation order: the rank of t among the group's members
-    const bool mine = ok[t] && lead[t] == l;
-    const unsigned bal = __ballot_sync(0xffffffffu, mine);
-    const int lane = t & 31;
-    if (lane == 0) cnt[sl][t >> 5] = __popc(bal);
-    asm volatile("bar.sync %0, %1;" ::"r"(1 + sl), "r"(SEG) : "memory");  // this slice's two warps
-    if (mine) T.member[__popc(bal & ((1u << lane) - 1u)) + ((t >> 5) ? cnt[sl][0] : 0)] = e;
-    if (t == 0) {
-      int lo = 1 << 30, hi = 0;
-      for (int u = 0; u < SEG; u++)
-        if (ok[u] && lead[u] == l) {
-          lo = min(lo, b.prep[start + u].i_lo);
-          hi = max(hi, b.prep[start + u].i_hi);
-        }
-      T.nmem = cnt_l[l];
+    const unsigned m0 = __ballot_sync(0xffffffffu, ok[lane] && lead[lane] == l);
+    const unsigned m1 = __ballot_sync(0xffffffffu, ok[lane + 32] && lead[lane + 32] == l);
+    const unsigned below = (1u << lane) - 1u;  // members in evaluation order
+    if (m0 >> lane & 1u) T.member[__popc(m0 & below)] = start + lane;
+    if (m1 >> lane & 1u) T.member[__popc(m0) + __popc(m1 & below)] = start + lane + 32;
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0) {
+      T.nmem = cnt[l];
       T.lo = lo;
       T.hi = hi;
     }
-    asm volatile("bar.sync %0, %1;" ::"r"(1 + sl), "r"(SEG) : "memory");  // cnt[sl] is reused
   }
-  __syncthreads();
-  const int lane = tid & 31, wsl = t >> 5;  // warp within the slice
-  for (int base = 0; base < ng; base += GROUP_SLICES) {
-    const int g = base + sl;
-    const bool act = g < ng;
-    if (t < GROUP_MAX) mem[sl][t] = -1;
-    __syncthreads();
-    if (act && gid[t] == g) mem[sl][slot[t]] = e;
-    __syncthreads();
-    GroupRec &R = b.grec[(size_t)start + (act ? g : 0)];
-    int c = -1, nm = 0;
-    float f = 0.0f, w[GROUP_MAX], wf[GROUP_MAX];
-    unsigned bal = 0u;
-    bool keep = false;
-    if (act) {
-      for (int m = 0; m < GROUP_MAX; m++) nm += mem[sl][m] >= 0;
-      // row t of the group: kept when any member weighs it
-      c = b.prep[mem[sl][0]].cols[t];
-      f = c >= 0 ? G.factor[c] : 0.0f;
-#pragma unroll
-      for (int m = 0; m < GROUP_MAX; m++) {
-        w[m] = (mem[sl][m] >= 0 && c >= 0) ? b.prep[mem[sl][m]].w[t] : 0.0f;
-        wf[m] = w[m] * f;
-        keep |= wf[m] != 0.0f;
-      }
-      bal = __ballot_sync(0xffffffffu, keep);
-      if (lane == 0) cnt[sl][wsl] = __popc(bal);
-    }
-    __syncthreads();
-    if (act) {
-      const int pos = __popc(bal & ((1u << lane) - 1u)) + (wsl ? cnt[sl][0] : 0);
-      if (keep) {
-        R.wf[pos][0] = make_float4(wf[0], wf[1], wf[2], wf[3]);
-        R.wf[pos][1] = make_float4(wf[4], wf[5], wf[6], wf[7]);
-        R.w[pos][0] = make_float4(w[0], w[1], w[2], w[3]);
-        R.w[pos][1] = make_float4(w[4], w[5], w[6], w[7]);
-        R.col[pos] = c;
-        R.f[pos] = f;
-      }
-      const int kept = cnt[sl][0] + cnt[sl][1];
-      const int padded = (kept + 7) & ~7;
-      if (t >= kept && t < padded) {  // zero-weight padding rows (add exactly 0)
-        const float4 z4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        R.wf[t][0] = R.wf[t][1] = R.w[t][0] = R.w[t][1] = z4;
-        R.col[t] = 0;
-        R.f[t] = 0.0f;
-      }
-      if (t < GROUP_MAX) R.member[t] = mem[sl][t];
-      if (t == 0) {
-        R.nmem = nm;
-        R.nn = padded;
-      }
-    }
-    __syncthreads();
-  }
+  for (int g = warp; g < ng; g += GROUP_W) write_group(G, b, b.grec[(size_t)start + g], mem[g], lane);
 }
 
-// One 64-thread CTA per listed table slot (two or more evaluations alone in
-// their segments chose it): the evaluations whose columns equal the first
-// one's (a hash collision leaves the others alone) become group records of
-// up to GROUP_MAX members like k_group's (rows any member weighs, in
-// reference order), and their own single-member records are switched off
-// (nmem 0).
-__global__ void __launch_bounds__(SEG) k_merge(DevGrid G, EvalBatch b) {
-  __shared__ int mem[MERGE_CAP];
-  __shared__ int nmem_s, cnt[2];
-  const int t = threadIdx.x, lane = t & 31, wv = t >> 5;
-  static_assert(MERGE_CAP == SEG, "one thread per listed evaluation");
+// One warp per listed table slot (two or more evaluations alone in their
+// segments chose it): the evaluations with the first one's columns become
+// group records of up to GROUP_MAX members, and their own single-member
+// records are switched off (nmem 0).
+constexpr int MERGE_W = 4;
+__global__ void __launch_bounds__(32 * MERGE_W) k_merge(DevGrid G, EvalBatch b) {
+  __shared__ int mem[MERGE_W][MERGE_CAP + GROUP_MAX];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nlist = b.mslot[0];
-  for (int j = blockIdx.x; j < nlist; j += gridDim.x) {
-    const int slot = b.mslot[1 + j];
-    const int nc = min(b.mcnt[slot], MERGE_CAP);
-    int e = -1;
-    if (t < nc) {
-      e = b.mmem[(size_t)slot * MERGE_CAP + t];
-      const int *c0 = b.prep[b.mmem[(size_t)slot * MERGE_CAP]].cols, *c = b.prep[e].cols;
-      bool same = true;
-      for (int n = 0; n < 64 && same; n++) same = c[n] == c0[n];
-      if (!same) e = -1;
+  for (int j = blockIdx.x * MERGE_W + warp; j < nlist; j += gridDim.x * MERGE_W) {
+    const int slot = b.mslot[1 + j], nc = min(b.mcnt[slot], MERGE_CAP);
+    const int *list = b.mmem + (size_t)slot * MERGE_CAP;
+    const int e0 = list[0];
+    int nt = 0;  // the matching evaluations, in list order
+    for (int i = lane; i < MERGE_CAP; i += 32) {
+      const int e = i < nc ? list[i] : -1;
+      const bool same = e >= 0 && same_cols(G, b, e0, b.prep[e0].key, e, b.prep[e].key);
+      const unsigned bal = __ballot_sync(0xffffffffu, same);
+      if (same) mem[warp][nt + __popc(bal & ((1u << lane) - 1u))] = e;
+      nt += __popc(bal);
     }
-    // compact the matching evaluations, keeping their order
-    const unsigned bm = __ballot_sync(0xffffffffu, e >= 0);
-    if (lane == 0) cnt[wv] = __popc(bm);
-    __syncthreads();
-    if (e >= 0) mem[__popc(bm & ((1u << lane) - 1u)) + (wv ? cnt[0] : 0)] = e;
-    if (t == 0) nmem_s = cnt[0] + cnt[1];
-    __syncthreads();
-    const int nt = nmem_s;
-    if (nt >= 2) {
+    if (lane < GROUP_MAX) mem[warp][nt + lane] = -1;
+    __syncwarp();
+    if (nt >= 2)
       for (int g0 = 0; g0 < nt; g0 += GROUP_MAX) {
-        const int nm = min(GROUP_MAX, nt - g0);
-        __shared__ int rec;
-        if (t == 0) rec = atomicAdd(b.mrcount, 1);
-        __syncthreads();
-        GroupRec &R = b.mrec[rec];
-        // row t of the group: kept when any member weighs it
-        const int c = b.prep[mem[g0]].cols[t];
-        const float f = c >= 0 ? G.factor[c] : 0.0f;
-        float w[GROUP_MAX], wf[GROUP_MAX];
-        bool keep = false;
-#pragma unroll
-        for (int m = 0; m < GROUP_MAX; m++) {
-          w[m] = (m < nm && c >= 0) ? b.prep[mem[g0 + m]].w[t] : 0.0f;
-          wf[m] = w[m] * f;
-          keep |= wf[m] != 0.0f;
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, keep);
-        __syncthreads();  // cnt is reused
-        if (lane == 0) cnt[wv] = __popc(bal);
-        __syncthreads();
-        const int pos = __popc(bal & ((1u << lane) - 1u)) + (wv ? cnt[0] : 0);
-        if (keep) {
-          R.wf[pos][0] = make_float4(wf[0], wf[1], wf[2], wf[3]);
-          R.wf[pos][1] = make_float4(wf[4], wf[5], wf[6], wf[7]);
-          R.w[pos][0] = make_float4(w[0], w[1], w[2], w[3]);
-          R.w[pos][1] = make_float4(w[4], w[5], w[6], w[7]);
-          R.col[pos] = c;
-          R.f[pos] = f;
-        }
-        const int kept = cnt[0] + cnt[1];
-        const int padded = (kept + 7) & ~7;
-        if (t >= kept && t < padded) {  // zero-weight padding rows (add exactly 0)
-          const float4 z4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          R.wf[t][0] = R.wf[t][1] = R.w[t][0] = R.w[t][1] = z4;
-          R.col[t] = 0;
-          R.f[t] = 0.0f;
-        }
-        if (t < GROUP_MAX) R.member[t] = t < nm ? mem[g0 + t] : -1;
-        if (t == 0) {
-          R.nmem = nm;
-          R.nn = padded;
-        }
-        if (t < nm) b.grec[b.erec[mem[g0 + t]]].nmem = 0;  // interpolated here instead
-        __syncthreads();
+        int rec = 0;
+        if (lane == 0) rec = atomicAdd(b.mrcount, 1);
+        rec = __shfl_sync(0xffffffffu, rec, 0);
+        write_group(G, b, b.mrec[rec], mem[warp] + g0, lane);
+        if (lane < GROUP_MAX && g0 + lane < nt) b.grec[b.erec[mem[warp][g0 + lane]]].nmem = 0;  // interpolated here instead
       }
-    }
-    __syncthreads();
+    __syncwarp();
   }
 }
 
@@ -345,10 +289,10 @@ void launch_group(const DevGrid &G, const EvalBatch &b, cudaStream_t s) {
     cudaMemsetAsync(b.mslot, 0, sizeof(int), s);
     cudaMemsetAsync(b.mrcount, 0, sizeof(int), s);
   }
-  k_group<<<num_segments(b), SEG * GROUP_SLICES, 0, s>>>(G, b);
+  k_group<<<num_segments(b), GROUP_T, 0, s>>>(G, b);
   count_launch();
   if (b.mkey) {
-    k_merge<<<num_sms() * 8, SEG, 0, s>>>(G, b);
+    k_merge<<<num_sms() * 4, 32 * MERGE_W, 0, s>>>(G, b);
     count_launch();
   }
 }

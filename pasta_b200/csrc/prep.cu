@@ -6,6 +6,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "device.cuh"
 #include "fft.cuh"
 #include "kernels.h"
 
@@ -33,24 +34,104 @@ __device__ __forceinline__ double index_of(const DevGrid &G, const DevStar &st, 
   return float_index_nonuni(G.wl_vals, G.npx, wl * P.shift_factor);
 }
 
-// One thread per evaluation: neighbours + weights (interpolate.rs:930-949),
-// rotation width and its error checks (convolve_rv.rs:484-519), the RV
-// range checks (convolve_rv.rs:547-567) and the pixel windows every later
-// stage works on.
-__global__ void k_prep(DevGrid G, EvalBatch b, int full_window) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+// local_grid by the PREP_L lanes of one evaluation: the nine independent
+// factor sets (4 teff rows, 4 logg columns, [M/H]) on a lane each, then lane l
+// writes the four neighbours of (teff neighbour l / 4, logg neighbour l % 4).
+// Same expressions, same values.
+constexpr int PREP_L = 16, PREP_T = 128;
+__device__ __forceinline__ int prep_neighbors(const GridGeom &G, double t, double m, double lg, int l, unsigned lanes,
+                                              EvalPrep &P) {
+  if (t != t || m != m || lg != lg) return S_NAN;
+  if (!teff_logg_ok(G, t, lg)) return S_OUT_OF_GRID;
+  if (!m_ok(G, m)) return S_OUT_OF_GRID;
+  int tlo, thi, llo, lhi;
+  int st = teff_index_limits_at(G, lg, tlo, thi);
+  if (st) return st;
+  st = logg_index_limits_at(G, t, llo, lhi);
+  if (st) return st;
+  int tn[4], mn[4], ln[4];
+  if (find_neighbors(G.tv, G.nt, t, tlo, thi, tn)) return S_NEIGHBORS;
+  if (find_neighbors(G.mv, G.nm, m, 0, G.nm - 1, mn)) return S_NEIGHBORS;
+  if (find_neighbors(G.lv, G.nl, lg, llo, lhi, ln)) return S_NEIGHBORS;
+  int ok = 0, mmask = 0;  // bit r*4+c; bit k
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    if (mn[c] >= 0) mmask |= 1 << c;
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+      if (tn[c] >= 0 && ln[r] >= 0 && ln[r] >= G.llo[tn[c]] && ln[r] <= G.lhi[tn[c]]) ok |= 1 << (r * 4 + c);
+  }
+  // lane l < 4: teff factors along logg row l; 4..7: logg factors down teff
+  // column l - 4; 8: [M/H] factors
+  double o[4] = {0.0, 0.0, 0.0, 0.0}, val[4];
+  int mask = mmask;
+  if (l < 4) mask = (ok >> (l * 4)) & 15;
+  else if (l < 8) mask = ((ok >> (l - 4)) & 1) | ((ok >> (l - 1)) & 2) | ((ok >> (l + 2)) & 4) | ((ok >> (l + 5)) & 8);
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int at = l < 4 ? tn[i] : l < 8 ? ln[i] : mn[i];
+    const double *v = l < 4 ? G.tv : l < 8 ? G.lv : G.mv;
+    val[i] = at >= 0 ? v[at] : 0.0;
+  }
+  const double x = l < 4 ? t : l < 8 ? lg : m;
+  if (l > 8) mask = 0;
+  if (__any_sync(lanes, coeffs_from_neighbors(x, mask, val, o) != 0)) return S_NEIGHBORS;
+  const int c = l >> 2, r = l & 3;
+  double ft = 0.0, fl = 0.0;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const double a = __shfl_sync(lanes, o[i], r, PREP_L), b = __shfl_sync(lanes, o[i], 4 + c, PREP_L);
+    if (i == c) ft = a;
+    if (i == r) fl = b;
+  }
+  const double a = ft * fl;
+  const bool pres = (ok >> (r * 4 + c)) & 1;
+  const int tc = c == 0 ? tn[0] : c == 1 ? tn[1] : c == 2 ? tn[2] : tn[3];
+  const int lr = r == 0 ? ln[0] : r == 1 ? ln[1] : r == 2 ? ln[2] : ln[3];
+  const int64_t col0 = pres ? (G.cum[tc] + lr - G.llo[tc]) * (int64_t)G.nm : 0;
+  int cols[4];
+  float w[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    w[k] = (float)(a * __shfl_sync(lanes, o[k], 8, PREP_L));
+    cols[k] = pres && mn[k] >= 0 ? (int)(col0 + mn[k]) : -1;
+  }
+  reinterpret_cast<int4 *>(P.cols)[l] = make_int4(cols[0], cols[1], cols[2], cols[3]);
+  reinterpret_cast<float4 *>(P.w)[l] = make_float4(w[0], w[1], w[2], w[3]);
+  if (l == 0)
+    P.key = (unsigned long long)(ok | mmask << 16) | (unsigned long long)(tn[1] & (AXIS_KEY - 1)) << 20 |
+            (unsigned long long)(ln[1] & (AXIS_KEY - 1)) << 34 | (unsigned long long)(mn[1] & (AXIS_KEY - 1)) << 48 |
+            1ull << 62;
+  return S_OK;
+}
+
+// PREP_L lanes per evaluation: neighbours + weights (interpolate.rs:930-949),
+// then on one lane the rotation width and its error checks
+// (convolve_rv.rs:484-519), the RV range checks (convolve_rv.rs:547-567) and
+// the pixel windows every later stage works on.  A chain of dependent reads
+// and double divisions: one thread per evaluation with the axes in global
+// memory took 17-34 us whatever the batch; 12-16 us with the axes in shared
+// memory and the factor sets side by side.
+__global__ void __launch_bounds__(PREP_T) k_prep(DevGrid G, EvalBatch b, int full_window) {
+  __shared__ double geo[GEOM_SMEM / 8];
+  const GridGeom GG = geom_shared(G.g, geo);
+  const int e = blockIdx.x * (PREP_T / PREP_L) + threadIdx.x / PREP_L, l = threadIdx.x % PREP_L;
   if (e >= b.E) return;
   EvalPrep &P = b.prep[e];
   const int s = b.eval_star[e];
-  P.star = s;
   if (b.eval_active && !b.eval_active[e]) {
-    P.status = S_INACTIVE;
+    if (l == 0) {
+      P.star = s;
+      P.status = S_INACTIVE;
+    }
     return;
   }
   const double *L = b.labels + 5 * (size_t)e;
   const DevStar &st = b.stars[s];
   const int N = G.npx;
-  int status = local_grid(G.g, L[0], L[1], L[2], P.cols, P.w);
+  int status = prep_neighbors(GG, L[0], L[1], L[2], l, 0xFFFFu << (threadIdx.x & 16), P);
+  if (l) return;
+  P.star = s;
   const double vsini = L[3], rv = L[4];
   P.vsini = vsini;
   int m = 1;
@@ -213,13 +294,13 @@ __global__ void __launch_bounds__(FFT_T) k_rotker(DevGrid G, EvalBatch b, const 
 void launch_prep(const DevGrid &G, const EvalBatch &b, cudaStream_t s) {
   if (b.E <= 0) return;
   if (b.direct_max > 0 && b.direct_count) cudaMemsetAsync(b.direct_count, 0, sizeof(int), s);
-  k_prep<<<(b.E + 127) / 128, 128, 0, s>>>(G, b, 0);
+  k_prep<<<(b.E + PREP_T / PREP_L - 1) / (PREP_T / PREP_L), PREP_T, 0, s>>>(G, b, 0);
   count_launch();
 }
 void launch_prep_full(const DevGrid &G, const EvalBatch &b, cudaStream_t s) {
   if (b.E <= 0) return;
   if (b.direct_max > 0 && b.direct_count) cudaMemsetAsync(b.direct_count, 0, sizeof(int), s);
-  k_prep<<<(b.E + 127) / 128, 128, 0, s>>>(G, b, 1);
+  k_prep<<<(b.E + PREP_T / PREP_L - 1) / (PREP_T / PREP_L), PREP_T, 0, s>>>(G, b, 1);
   count_launch();
 }
 void launch_rotker(const DevGrid &G, const EvalBatch &b, const float2 *tw, cudaStream_t s) {
@@ -272,6 +353,8 @@ __device__ int block_min_int(int v, int *sm) {
 // evaluation just publish their host-placed positions.
 __global__ void __launch_bounds__(MAX_PARTICLES) k_pso_update(DevGrid G, Swarm W) {
   __shared__ int sm[MAX_PARTICLES];
+  __shared__ double geo[GEOM_SMEM / 8];
+  const GridGeom GG = geom_shared(G.g, geo);
   const int s = blockIdx.x, p = threadIdx.x;
   const PsoParams &S = W.params[s];
   const bool star_ok = W.active[s] && !W.done[s] && W.status[s] == 0;
@@ -301,10 +384,10 @@ __global__ void __launch_bounds__(MAX_PARTICLES) k_pso_update(DevGrid G, Swarm W
         for (int k = 0; k < 5; k++) nx[k] = xx[k];
         nx[d] += vv[d];
         double c;
-        int st = pso_clamp_1d(G.g, S, nx, d, c);
+        int st = pso_clamp_1d(GG, S, nx, d, c);
         if (st) { err = st; break; }
         xx[d] = c;
-        if (!pso_within(G.g, S, xx)) { err = S_BOUNDS; break; }
+        if (!pso_within(GG, S, xx)) { err = S_BOUNDS; break; }
       }
       if (!err) {
         for (int d = 0; d < 5; d++) {

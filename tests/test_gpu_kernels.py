@@ -119,3 +119,41 @@ def test_resampling_of_broadening_blocks(env, n_obs, vsini, rv):
     ref, st = O.chi2(og, od, oc, flux, var, lab, O.F64)
     assert st[0] == 0
     assert abs(got - ref[0]) <= CHI2_TOL * ref[0]
+
+
+def _contracted(star, n, seed):
+    rng = np.random.default_rng(seed)
+    return star.label + rng.uniform(-1.0, 1.0, (n, 5)) * [20.0, 0.004, 0.01, 5.0, 1.0]
+
+
+@pytest.mark.parametrize("members", [8, 17, 64])
+def test_tensor_core_groups_alone_and_among_many(env, members):
+    """One tensor-core group is cut into items of two tiles, hundreds of groups into whole slabs; every pixel is the same."""
+    P, star, interp = env["P"], env["star"], env["interp"]
+    disp = P.FixedResolutionDispersion(star.wl, 85000.0, env["wl"])
+    keep = interp.tc_min
+    try:
+        interp.tc_min = 8
+        lab = _contracted(star, 64 * 640, 8)
+        lab[members:64] = _near(star, 64 - members, 9)  # the first segment's group has `members` evaluations
+        fitter = interp.get_fitter(disp, P.ConstantContinuum(), P.PSOSettings(8, 2), (0.0, 300.0), (-150.0, 150.0))
+        many = np.array(fitter.chi2(interp, star.flux, star.var, lab))
+        few = np.array(fitter.chi2(interp, star.flux, star.var, lab[:64]))
+    finally:
+        interp.tc_min = keep
+    np.testing.assert_array_equal(many[:64], few)
+
+
+def test_groups_at_grid_edges(env):
+    """Evaluations of one segment whose cubes lie at the grid's edges and nodes (two or three neighbours on an axis):
+    together, in any group, as one at a time."""
+    P, spec, interp = env["P"], env["spec"], env["interp"]
+    rng = np.random.default_rng(12)
+
+    def axis(v):
+        return rng.choice(np.concatenate([v[[0, 1, -2, -1]], v[[0, 0, -2, -2]] + rng.uniform(0.2, 0.8, 4) * np.diff(v)[[0, 0, -1, -1]]]))
+    lab = np.array([[axis(spec.teffs), axis(spec.ms), axis(spec.loggs)] for _ in range(150)])
+    lab[100:] = lab[rng.integers(0, 100, 50)]  # shared cubes
+    together = interp.interpolate_bulk(lab)
+    for i in list(range(0, 150, 7)) + [149]:
+        np.testing.assert_array_equal(together[i], interp.interpolate(*lab[i]))
