@@ -695,7 +695,7 @@ class _Interpolator:
         check(lib().pasta_chi2_many(self._grid._h, S, dh, ch, fp, vp, ptr(n), ptr(lab), ptr(out), ptr(st)))
         if not allow_nan:
             self._raise_status(st, "chi2")
-        return [float(x) for x in out]
+        return out.tolist()
 
     def ccf(self, vs, teff, m, logg, dispersion, observed_flux) -> np.ndarray:
         """Cross-correlation of the unbroadened model with the flux (lib.rs:1340-1371)."""
@@ -949,7 +949,7 @@ class SingleFitter:
                                ptr(vr), len(fl), ptr(lab), len(lab), ptr(out), ptr(st)))
         if allow_nan is False:
             _Interpolator._raise_status(st, "chi2")
-        return [float(x) for x in out]
+        return out.tolist()
 
 
     def compute_uncertainty(self, interpolator, observed_flux, observed_var, spec_res: float, label,
@@ -1060,7 +1060,7 @@ class BinaryFitter:
                                       ptr(out), ptr(st)))
         if allow_nan is False:
             _Interpolator._raise_status(st, "chi2")
-        return [float(x) for x in out]
+        return out.tolist()
 
 
 def _write_trace(tr, trace_directory, best_particle_file):

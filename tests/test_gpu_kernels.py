@@ -157,3 +157,39 @@ def test_groups_at_grid_edges(env):
     together = interp.interpolate_bulk(lab)
     for i in list(range(0, 150, 7)) + [149]:
         np.testing.assert_array_equal(together[i], interp.interpolate(*lab[i]))
+
+
+@pytest.mark.parametrize("n", [1, 300, 349, 350, 1100])
+def test_results_copied_in_parts(env, n):
+    """Model rows copied out through the staging buffer's halves of 4 MB (349 rows of 3,001 pixels just fit one):
+    less than a half, a half, one row more, several."""
+    P, star, interp = env["P"], env["star"], env["interp"]
+    disp = P.FixedResolutionDispersion(star.wl, 85000.0, env["wl"])
+    lab = _near(star, n, 31)
+    many = interp.produce_model_bulk(disp, lab)
+    for i in {0, n // 2, n - 1, min(n - 1, 348), min(n - 1, 349)}:
+        np.testing.assert_array_equal(many[i], interp.produce_model(disp, *lab[i]))
+
+
+def test_calls_from_several_threads(env):
+    """Calls of several threads on one grid share the scratch memory and the staging buffer; every result is its own."""
+    import threading
+    P, star, interp = env["P"], env["star"], env["interp"]
+    disp = P.FixedResolutionDispersion(star.wl, 85000.0, env["wl"])
+    fitter = interp.get_fitter(disp, P.ChunkContinuumFitter(star.wl, 5, 8, 0.2), P.PSOSettings(8, 2), (0.0, 300.0),
+                               (-150.0, 150.0))
+    labs = [_near(star, 20 + 37 * k, k) for k in range(6)]
+    want = [(np.array(fitter.chi2(interp, star.flux, star.var, lab)), interp.produce_model_bulk(disp, lab)) for lab in labs]
+    bad = []
+
+    def work(k):
+        for _ in range(10):
+            c, m = np.array(fitter.chi2(interp, star.flux, star.var, labs[k])), interp.produce_model_bulk(disp, labs[k])
+            if not (np.array_equal(c, want[k][0]) and np.array_equal(m, want[k][1])):
+                bad.append(k)
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
