@@ -38,6 +38,17 @@ int num_sms() {
   return g_num_sms;
 }
 
+// Asynchronous 16-byte global -> shared copies (cp.async): the next tile's
+// input streams in while the current one is worked.  A copy with ok ==
+// false reads nothing and fills zeros.
+__device__ __forceinline__ void cp_async16(float *smem, const float *gmem, bool ok) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  const int n = ok ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(gmem), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+
 // ---------------------------------------------------------------- interp
 // flux[px] = sum_n w_n * u16_n[px] * factor_n over the 64 neighbours
 // (interpolate.rs:954-981).  Particles of one star soon sit in the same grid
@@ -119,7 +130,12 @@ __device__ __forceinline__ void write_group(const DevGrid &G, const EvalBatch &b
     R.col[pos] = 0;
     R.f[pos] = 0.0f;
   }
-  if (lane < GROUP_MAX) R.member[lane] = mem[lane];
+  if (lane < GROUP_MAX) {
+    const int m = mem[lane];
+    R.member[lane] = m;
+    R.lo[lane] = m >= 0 ? b.prep[m].i_lo : 0;
+    R.hi[lane] = m >= 0 ? b.prep[m].i_hi : 0;
+  }
   if (lane == 0) {
     R.nmem = nm;
     R.nn = padded;
@@ -309,12 +325,9 @@ __device__ __forceinline__ float grp_w(const float4 (&v)[2], int m) {
 // the NM members of a group on this thread's 4 pixels (one 64-bit load per row)
 template <int NM>
 __device__ __forceinline__ void interp_members(const DevGrid &G, const EvalBatch &b, const GroupRec &R, int px) {
-  // member m's window holds px (re-evaluated at the stores, so that the
-  // members' indices need no registers across the row loop)
-  auto inside = [&](int m) {
-    const EvalPrep &P = b.prep[R.member[m]];
-    return px >= P.i_lo && px < P.i_hi;
-  };
+  // member m's window holds px (read again at the stores, so that the windows
+  // need no registers across the row loop)
+  auto inside = [&](int m) { return px >= R.lo[m] && px < R.hi[m]; };
   bool any = false;
 #pragma unroll
   for (int m = 0; m < NM; m++) any |= inside(m);
@@ -325,7 +338,7 @@ __device__ __forceinline__ void interp_members(const DevGrid &G, const EvalBatch
 #pragma unroll
     for (int m = 0; m < NM; m++) acc[m][0] = acc[m][1] = make_float2(0.0f, 0.0f);
     const float2 bias = make_float2(-8388608.0f, -8388608.0f);
-    constexpr int UNR = NM > 4 ? 4 : NM > 2 ? 8 : 16;  // row loads in flight per thread (with their weights in registers)
+    constexpr int UNR = NM > 4 ? 4 : 8;  // row loads in flight per thread (with their weights in registers)
 #pragma unroll UNR
     for (int n = 0; n < nn; n++) {
       const uint2 q = __ldg(reinterpret_cast<const uint2 *>(G.spectra + (size_t)R.col[n] * G.stride + px));
@@ -392,71 +405,77 @@ __device__ __forceinline__ void interp_group(const DevGrid &G, const EvalBatch &
   }
 }
 
+// group record -> shared memory, 16 bytes per copy, not waited for
+__device__ __forceinline__ void rec_load(GroupRec *dst, const GroupRec *src) {
+  static_assert(sizeof(GroupRec) % 16 == 0, "16-byte copies");
+  const float *s = reinterpret_cast<const float *>(src);
+  float *d = reinterpret_cast<float *>(dst);
+  for (int i = threadIdx.x; i < (int)(sizeof(GroupRec) / 16); i += IT_T) cp_async16(d + 4 * i, s + 4 * i, true);
+}
+
 // Grid: x = segment, y = tile of IT_TILE pixels, so CTAs that run together read
 // the same tile slab of the resident grid (57 MB for 13,860 x 80,000), which
 // stays in L2; z = slice of the segment's groups (groups z, z + Z, ...), more
 // than one only for batches too small to fill the GPU otherwise.  Groups have
-// disjoint members, so the slicing does not change any result.
-__global__ void __launch_bounds__(IT_T, 3) k_interp(DevGrid G, EvalBatch b) {
-  __shared__ GroupRec R;
+// disjoint members, so the slicing does not change any result.  The next
+// record is copied in while the rows of one are read (one barrier a group);
+// its members' windows come with it.  Bound by instruction issue (67%: the
+// u16 -> f32 conversions) and the rows' L2 latency: 2,500 evaluations spread
+// over 13,860 x 80,000 models, alone and merged: 599 + 795 us with the record
+// and the windows read between two barriers at 3 CTAs per SM (80 registers),
+// 503 + 822 us with the copy ahead, 490 + 714 us at 4 CTAs (64 registers, 24
+// bytes spilled by the largest groups); 2 rows in flight for those instead
+// of 4: 478 + 947.
+__global__ void __launch_bounds__(IT_T, 4) k_interp(DevGrid G, EvalBatch b) {
+  __shared__ GroupRec R[2];
   const int s = blockIdx.x;
   const int px = blockIdx.y * IT_TILE + threadIdx.x * IT_PX;
   const int ng = b.gcount[s];
   int start, len;
   seg_range(b, s, start, len);
-  for (int g = blockIdx.z; g < ng; g += gridDim.z) {
-    const float4 *src = reinterpret_cast<const float4 *>(b.grec + (size_t)start + g);
-    float4 *dst = reinterpret_cast<float4 *>(&R);
-    for (int i = threadIdx.x; i < (int)(sizeof(GroupRec) / 16); i += IT_T) dst[i] = src[i];
-    __syncthreads();
-    interp_group(G, b, R, px);
-    __syncthreads();
+  const GroupRec *rec = b.grec + start;
+  int k = 0;
+  if ((int)blockIdx.z < ng) rec_load(&R[0], rec + blockIdx.z);
+  for (int g = blockIdx.z; g < ng; g += gridDim.z, k ^= 1) {
+    cp_async_commit();
+    cp_async_wait_all();
+    __syncthreads();  // this record is here, and the other buffer is no longer read
+    if (g + (int)gridDim.z < ng) rec_load(&R[k ^ 1], rec + g + gridDim.z);
+    interp_group(G, b, R[k], px);
   }
 }
 
 // Groups merged across segments (k_merge), in work items (record, tile)
 // taken tile by tile, so that CTAs that run together read the same tile
 // slab of the grid; their number is known on the device only.
-__global__ void __launch_bounds__(IT_T, 3) k_interp_merged(DevGrid G, EvalBatch b) {
-  __shared__ GroupRec R;
+__global__ void __launch_bounds__(IT_T, 4) k_interp_merged(DevGrid G, EvalBatch b) {
+  __shared__ GroupRec R[2];
   const int nrec = *b.mrcount;
   const long long work = (long long)nrec * ((G.npx + IT_TILE - 1) / IT_TILE);
-  for (long long w = blockIdx.x; w < work; w += gridDim.x) {
-    const int tile = (int)(w / nrec), rec = (int)(w - (long long)tile * nrec);
-    const float4 *src = reinterpret_cast<const float4 *>(b.mrec + rec);
-    float4 *dst = reinterpret_cast<float4 *>(&R);
-    for (int i = threadIdx.x; i < (int)(sizeof(GroupRec) / 16); i += IT_T) dst[i] = src[i];
+  int k = 0;
+  if (blockIdx.x < work) rec_load(&R[0], b.mrec + blockIdx.x % nrec);
+  for (long long w = blockIdx.x; w < work; w += gridDim.x, k ^= 1) {
+    cp_async_commit();
+    cp_async_wait_all();
     __syncthreads();
-    interp_group(G, b, R, tile * IT_TILE + threadIdx.x * IT_PX);
-    __syncthreads();
+    if (w + gridDim.x < work) rec_load(&R[k ^ 1], b.mrec + (w + gridDim.x) % nrec);
+    interp_group(G, b, R[k], (int)(w / nrec) * IT_TILE + threadIdx.x * IT_PX);
   }
 }
 
 void launch_interp(const DevGrid &G, const EvalBatch &b, cudaStream_t s) {
   if (b.E <= 0) return;
   const int segs = num_segments(b), tiles = (G.npx + IT_TILE - 1) / IT_TILE;
-  const int want = num_sms() * 6;  // two waves of the 3 CTAs an SM holds
+  const int want = num_sms() * 8;  // two waves of the 4 CTAs an SM holds
   const int z = segs * tiles >= want ? 1 : std::min(SEG, (want + segs * tiles - 1) / (segs * tiles));
   dim3 grid(segs, tiles, z);
   k_interp<<<grid, IT_T, 0, s>>>(G, b);
   count_launch();
   if (b.mkey) {
-    k_interp_merged<<<num_sms() * 6, IT_T, 0, s>>>(G, b);
+    k_interp_merged<<<num_sms() * 8, IT_T, 0, s>>>(G, b);
     count_launch();
   }
 }
-
-// ------------------------------------------------------ fused broadening
-// Asynchronous 16-byte global -> shared copies (cp.async): the next tile's
-// input streams in while the current one is worked.  A copy with ok ==
-// false reads nothing and fills zeros.
-__device__ __forceinline__ void cp_async16(float *smem, const float *gmem, bool ok) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  const int n = ok ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(gmem), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
 // ----------------------------------------------- direct broadening (narrow)
 // Evaluations whose combined kernel (m rotation taps + 2 hg instrument taps)

@@ -19,6 +19,7 @@ struct __align__(16) GroupRec {
   int col[64];            // grid row of compacted neighbour n
   float f[64];            // its dequantisation factor
   int member[GROUP_MAX];  // evaluation indices (-1: unused)
+  int lo[GROUP_MAX], hi[GROUP_MAX];  // the members' interpolation windows (empty: unused)
   int nmem, nn;           // members, compacted rows
   int pad[2];
 };
