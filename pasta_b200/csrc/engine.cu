@@ -1870,8 +1870,9 @@ void tune_direct(pasta_grid *g) {
 // cores on this device and grid: 16 segments of 64 evaluations, each split
 // into groups of gs evaluations in distinct grid cubes, interpolated with
 // the tensor-core path on and off (CUDA events, best of 3 after a warm-up),
-// for gs on a ladder; the smallest gs at which the tensor cores win, and
-// every larger gs on the ladder, sets the threshold (SEG + 1: never).
+// for gs on a ladder; the smallest gs at which the tensor cores gain a sixth,
+// and still win at every larger gs on the ladder, sets the threshold (SEG + 1:
+// never).
 void tune_interp_tc(pasta_grid *g) {
   g->tc_min = 16;
   if (const char *ev = getenv("PASTA_INTERP_TC_MIN")) {
@@ -1958,10 +1959,10 @@ void tune_interp_tc(pasta_grid *g) {
     if (getenv("PASTA_TUNE_VERBOSE"))
       fprintf(stderr, "pasta_b200 tune: %lld px, groups of %d: CUDA cores %.4f ms, tensor cores %.4f ms\n",
               (long long)g->npx, gs, tm[0], tm[1]);
-    // a near-tie stays with the CUDA cores: the two forms round differently,
-    // and the choice should not vary from one process to the next
-    if (tm[1] < 0.95f * tm[0]) {
-      if (best > SEG) best = gs;
+    // the first size that gains a sixth: at a near-tie the choice would vary
+    // from one process to the next, and the two forms round differently
+    if (tm[1] < tm[0]) {
+      if (best > SEG && tm[1] < (5.0f / 6.0f) * tm[0]) best = gs;
     } else {
       best = SEG + 1;  // the tensor cores must win from the threshold on
     }

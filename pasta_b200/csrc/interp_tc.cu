@@ -29,7 +29,7 @@
 //               M = 128, N = members rounded up to 16) into one of ND
 //               tensor-memory accumulators;
 //   warps 2-9   converters: staging -> the bf16 byte planes of A (a ring of
-//               NA buffers), and each item's B (two buffers, so the next
+//               NA buffers in tensor memory), and each item's B (two buffers, so the next
 //               item's weights are written while the last tiles of the
 //               current one multiply);
 //   warps 10-13 epilogue: tcgen05.ld of an accumulator (warp w reads lanes
@@ -37,6 +37,14 @@
 // The last npx % 128 pixels carry the reference's extra 1/65535
 // (interpolate.rs:978) and are computed on the CUDA cores by the epilogue
 // warps.
+//
+// What bounds it: a tile's products, its conversion and its stores take about
+// as long as one another.  8,000 evaluations in groups of 64, 80,000 pixels
+// (ncu): 968 us with A in shared memory, the products issued by a single
+// thread and a row pointer read from shared memory before every store; 860 us
+// with the members read eight at a time, 830 us with A in tensor memory, 750
+// us with the issuing warp converged.  A second set of epilogue warps gains 3%
+// and spills; shuffles instead of the member table 850 us.
 //
 // Every wait on an mbarrier is bounded (about a second); a wait that runs
 // out marks the CTA's groups with an internal error, the other roles stop at
@@ -60,7 +68,10 @@ constexpr int NSTG = 4;            // staging ring (raw rows)
 constexpr int NA = 2;              // A ring
 constexpr int ND = 4;              // accumulators in tensor memory
 constexpr int DCOLS = 64;          // columns of an accumulator (members)
-constexpr int TMEM_COLS = ND * DCOLS;
+constexpr int ACOLS = TK / 2;        // tensor-memory columns of an A buffer (two bf16 each)
+constexpr int TMEM_A = ND * DCOLS;   // first column of the A ring
+constexpr int TMEM_COLS = 512;       // ND DCOLS + NA ACOLS, rounded up to a power of two
+static_assert(TMEM_A + NA * ACOLS <= TMEM_COLS, "tensor memory");
 constexpr int TSLAB = 64;          // tiles per item at most
 constexpr int S_TC_TIMEOUT = -99;  // PASTA_E_INTERNAL
 
@@ -69,24 +80,21 @@ constexpr int W_TMA = 0, W_MMA = 1, W_CV = 2, N_CV = 8, W_EP = W_CV + N_CV, N_EP
 constexpr int TT = 32 * (W_EP + N_EP);  // 448 threads
 constexpr int CVT = 32 * N_CV;          // converter threads
 
-// shared memory (bytes): staging ring [64 rows][128 pixels] u16, A ring
-// [128 pixels][128] bf16 (K-major), two B buffers of three parts
+// shared memory (bytes): staging ring [64 rows][128 pixels] u16, two B buffers of three parts
 // [64 members][64] bf16 (K-major), barriers, flags, the epilogue's member table
 constexpr int SZ_STG = 64 * TPX * 2;
-constexpr int SZ_A = TPX * TK * 2;
 constexpr int SZ_BP = 64 * BK * 2;
 constexpr int SB_STG = 0;
-constexpr int SB_A = SB_STG + NSTG * SZ_STG;
-constexpr int SB_B = SB_A + NA * SZ_A;
+constexpr int SB_B = SB_STG + NSTG * SZ_STG;
 constexpr int SB_BAR = SB_B + 2 * 3 * SZ_BP;
 // barrier indices
 constexpr int B_SFULL = 0, B_SEMPTY = B_SFULL + NSTG, B_AFULL = B_SEMPTY + NSTG, B_AEMPTY = B_AFULL + NA,
               B_DFULL = B_AEMPTY + NA, B_DEMPTY = B_DFULL + ND, B_BFULL = B_DEMPTY + ND, B_BEMPTY = B_BFULL + 2,
               B_DRAIN = B_BEMPTY + 2, NBAR = B_DRAIN + 1;
 constexpr int SB_MISC = SB_BAR + NBAR * 8;  // tensor-memory address, error flag
-constexpr int SB_EPI = (SB_MISC + 16 + 15) & ~15;  // per member: row pointer (8 B), window lo, hi
-constexpr int SB_TOTAL = SB_EPI + 64 * 16;
-static_assert(SB_A % 1024 == 0 && SB_B % 1024 == 0 && SB_BAR % 8 == 0, "shared layout");
+constexpr int SB_EPI = (SB_MISC + 16 + 15) & ~15;  // per member: evaluation, window lo, hi
+constexpr int SB_TOTAL = SB_EPI + 64 * 12;
+static_assert(SB_B % 1024 == 0 && SB_BAR % 8 == 0, "shared layout");
 static_assert(SB_TOTAL <= 227 * 1024, "shared memory of one CTA");
 
 // byte offset of element (row, k) of a K-major bf16 tile with KX elements
@@ -106,15 +114,36 @@ __device__ __forceinline__ uint64_t desc16(uint32_t saddr) {
 __device__ __forceinline__ uint32_t idesc_bf16(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
+// A in tensor memory (lane = row of A, two consecutive K elements per column)
+// issued by the lane with `one` set
+__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t acc,
+                                         uint32_t one) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-      "l"(da), "l"(db), "r"(idesc), "r"(acc));
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(db), "r"(idesc), "r"(acc), "r"(one));
 }
-__device__ __forceinline__ void mma_commit(uint32_t mbar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar)
-               : "memory");
+// 1 on one lane of the (converged) warp
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(r));
+  return r;
+}
+// 16 consecutive 32-bit columns of this thread's tensor-memory lane
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};\n" ::
+          "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+      "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void mma_commit(uint32_t mbar, uint32_t one) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(mbar),
+      "r"(one)
+      : "memory");
 }
 __device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(mbar), "r"(count) : "memory");
@@ -318,47 +347,51 @@ __global__ void __launch_bounds__(TT, 1) k_interp_tc(DevGrid G, EvalBatch b, con
     __syncwarp();
   } else if (w == W_MMA) {
     // ------------------------------------------------------------- MMA
-    if (lane == 0) {
-      long long g = 0;   // tiles multiplied
-      long long it = 0;  // items
-      for (int item = blockIdx.x; item < nitems && !*err; item += gridDim.x) {
-        TcItem I;
-        if (!tc_item(G, b, item, slabs, ts, I)) continue;
-        const int bb = (int)(it & 1);
-        if (!mbar_wait(bar(B_BFULL + bb), (uint32_t)((it >> 1) & 1))) *err = 1;
+    // The warp stays converged and one lane issues, so that the operands are
+    // warp-uniform (with the loop on one thread, moving them to uniform
+    // registers made a product of 128 x 64 x 16 take 85 cycles to issue).
+    const uint32_t one = elect_one();
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    long long g = 0;   // tiles multiplied
+    long long it = 0;  // items
+    bool stop = false;
+    for (int item = blockIdx.x; item < nitems && !stop; item += gridDim.x) {
+      TcItem I;
+      if (!tc_item(G, b, item, slabs, ts, I)) continue;
+      const int bb = (int)(it & 1);
+      stop = !warp_wait(bar(B_BFULL + bb), (uint32_t)((it >> 1) & 1), err);
+      tc_fence_after();
+      const uint32_t idesc = __shfl_sync(0xffffffffu, idesc_bf16(TPX, I.NP), 0);
+      const int nt = __shfl_sync(0xffffffffu, I.ntiles, 0);
+      for (int i = 0; i < nt && !stop; i++, g++) {
+        const int a = (int)(g % NA), d = (int)(g % ND);
+        stop = !warp_wait(bar(B_AFULL + a), (uint32_t)((g / NA) & 1), err);
+        if (!stop && g >= ND) stop = !warp_wait(bar(B_DEMPTY + d), (uint32_t)((g / ND - 1) & 1), err);
+        if (stop) break;
         tc_fence_after();
-        const uint32_t idesc = idesc_bf16(TPX, I.NP);
-        for (int i = 0; i < I.ntiles && !*err; i++, g++) {
-          const int a = (int)(g % NA), d = (int)(g % ND);
-          if (!mbar_wait(bar(B_AFULL + a), (uint32_t)((g / NA) & 1))) *err = 1;
-          if (g >= ND && !mbar_wait(bar(B_DEMPTY + d), (uint32_t)((g / ND - 1) & 1))) *err = 1;
-          if (*err) break;
-          tc_fence_after();
-          const uint64_t da = desc16<TK>(sbase + SB_A + (uint32_t)(a * SZ_A));
-          const uint32_t td = tmem + (uint32_t)(d * DCOLS);
+        const uint32_t ta = tm + (uint32_t)(TMEM_A + a * ACOLS), td = tm + (uint32_t)(d * DCOLS);
 #pragma unroll
-          for (int j = 0; j < 3; j++) {
-            const uint64_t db = desc16<BK>(sbase + SB_B + (uint32_t)((bb * 3 + j) * SZ_BP));
+        for (int j = 0; j < 3; j++) {
+          const uint64_t db = desc16<BK>(sbase + SB_B + (uint32_t)((bb * 3 + j) * SZ_BP));
 #pragma unroll
-            for (int ks = 0; ks < TK / 16; ks++)
-              mma_bf16(td, da + (uint64_t)((ks * 256) >> 4), db + (uint64_t)(((ks & 3) * 256) >> 4), idesc,
-                       (j | ks) ? 1u : 0u);
-          }
-          mma_commit(bar(B_AEMPTY + a));  // A slot free once these products have read it
-          mma_commit(bar(B_DFULL + d));   // accumulator ready
+          for (int ks = 0; ks < TK / 16; ks++)
+            mma_bf16(td, ta + (uint32_t)(ks * 8), db + (uint64_t)(((ks & 3) * 256) >> 4), idesc, (j | ks) ? 1u : 0u, one);
         }
-        mma_commit(bar(B_BEMPTY + bb));  // this item's weights are free
-        it++;
+        mma_commit(bar(B_AEMPTY + a), one);  // A slot free once these products have read it
+        mma_commit(bar(B_DFULL + d), one);   // accumulator ready
       }
-      // every product has completed before tensor memory is freed (bounded)
-      mma_commit(bar(B_DRAIN));
-      mbar_wait(bar(B_DRAIN), 0u);
+      mma_commit(bar(B_BEMPTY + bb), one);  // this item's weights are free
+      it++;
     }
+    // every product has completed before tensor memory is freed (bounded)
+    mma_commit(bar(B_DRAIN), one);
+    mbar_wait(bar(B_DRAIN), 0u);
     __syncwarp();
   } else if (w < W_EP) {
     // ------------------------------------------------------ converters
     const int c = t - 32 * W_CV;  // 0 .. CVT - 1
-    const int p = c & (TPX - 1), half = c >> 7;
+    // pixel p = tensor-memory lane; a warp reaches the lanes 32 (w % 4) ..
+    const int p = 32 * (w & 3) + lane, half = (w - W_CV) >> 2;
     long long g = 0, it = 0;
     bool stop = false;
     for (int item = blockIdx.x; item < nitems && !stop; item += gridDim.x) {
@@ -404,29 +437,27 @@ __global__ void __launch_bounds__(TT, 1) k_interp_tc(DevGrid G, EvalBatch b, con
         // A slot a: its products two tiles ago have completed
         stop = g >= NA ? !warp_wait(bar(B_AEMPTY + a), (uint32_t)((g / NA - 1) & 1), err) : false;
         if (stop) break;
-        unsigned char *A = sm + SB_A + a * SZ_A;
+        tc_fence_after();
+        uint32_t h[16], l[16];  // two rows each: 256 x high byte, low byte
 #pragma unroll
-        for (int k8 = 0; k8 < 32; k8 += 8) {
-          uint32_t h[4], l[4];
-#pragma unroll
-          for (int q = 0; q < 4; q++) {
-            const uint32_t u0 = u[k8 + 2 * q], u1 = u[k8 + 2 * q + 1];
-            // exact floats of the byte planes (below 2^23): f = bits(0x4B000000 | x) - 2^23
-            const float2 fh = __fadd2_rn(make_float2(__uint_as_float(0x4B000000u | (u0 & 0xFF00u)),
-                                                     __uint_as_float(0x4B000000u | (u1 & 0xFF00u))),
-                                         make_float2(-8388608.0f, -8388608.0f));
-            const float2 fl = __fadd2_rn(make_float2(__uint_as_float(0x4B000000u | (u0 & 0xFFu)),
-                                                     __uint_as_float(0x4B000000u | (u1 & 0xFFu))),
-                                         make_float2(-8388608.0f, -8388608.0f));
-            // at most 8 significant bits: the bf16 value is the top half of the f32
-            h[q] = __byte_perm(__float_as_uint(fh.x), __float_as_uint(fh.y), 0x7632);
-            l[q] = __byte_perm(__float_as_uint(fl.x), __float_as_uint(fl.y), 0x7632);
-          }
-          const int k = 32 * half + k8;
-          *reinterpret_cast<uint4 *>(A + kmaj16<TK>(p, k)) = make_uint4(h[0], h[1], h[2], h[3]);
-          *reinterpret_cast<uint4 *>(A + kmaj16<TK>(p, 64 + k)) = make_uint4(l[0], l[1], l[2], l[3]);
+        for (int q = 0; q < 16; q++) {
+          const uint32_t u0 = u[2 * q], u1 = u[2 * q + 1];
+          // exact floats of the byte planes (below 2^23): f = bits(0x4B000000 | x) - 2^23
+          const float2 fh = __fadd2_rn(make_float2(__uint_as_float(0x4B000000u | (u0 & 0xFF00u)),
+                                                   __uint_as_float(0x4B000000u | (u1 & 0xFF00u))),
+                                       make_float2(-8388608.0f, -8388608.0f));
+          const float2 fl = __fadd2_rn(make_float2(__uint_as_float(0x4B000000u | (u0 & 0xFFu)),
+                                                   __uint_as_float(0x4B000000u | (u1 & 0xFFu))),
+                                       make_float2(-8388608.0f, -8388608.0f));
+          // at most 8 significant bits: the bf16 value is the top half of the f32
+          h[q] = __byte_perm(__float_as_uint(fh.x), __float_as_uint(fh.y), 0x7632);
+          l[q] = __byte_perm(__float_as_uint(fl.x), __float_as_uint(fl.y), 0x7632);
         }
-        proxy_fence();
+        const uint32_t ta = tmem + ((uint32_t)(32 * (w & 3)) << 16) + (uint32_t)(TMEM_A + a * ACOLS + 16 * half);
+        tmem_st16(ta, h);
+        tmem_st16(ta + 32u, l);
+        tmem_wait_st();
+        tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(B_AFULL + a));
       }
@@ -435,8 +466,8 @@ __global__ void __launch_bounds__(TT, 1) k_interp_tc(DevGrid G, EvalBatch b, con
     // -------------------------------------------------------- epilogue
     const int e = t - 32 * W_EP;  // 0 .. 127
     const int q = w & 3;          // tensor-memory lanes 32 q .. 32 q + 31
-    float **rowp = reinterpret_cast<float **>(sm + SB_EPI);
-    int *wlo = reinterpret_cast<int *>(sm + SB_EPI + 64 * 8), *whi = wlo + 64;
+    int *mem = reinterpret_cast<int *>(sm + SB_EPI), *wlo = mem + 64, *whi = wlo + 64;
+    const unsigned row_bytes = (unsigned)b.stride * 4u;  // rows are far below 4 GB
     long long g = 0;
     bool stop = false;  // uniform within a warp; made uniform over the epilogue warps at each item
     for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
@@ -446,7 +477,7 @@ __global__ void __launch_bounds__(TT, 1) k_interp_tc(DevGrid G, EvalBatch b, con
       if (ep_any(stop || *err != 0)) break;
       if (e < 64) {
         const int m = e < I.nm ? I.R->member[e] : -1;
-        rowp[e] = m >= 0 ? b.bufA + (size_t)m * b.stride : b.bufA;
+        mem[e] = m >= 0 ? m : 0;
         wlo[e] = m >= 0 ? b.prep[m].i_lo : 0;
         whi[e] = m >= 0 ? b.prep[m].i_hi : 0;
       }
@@ -474,28 +505,32 @@ __global__ void __launch_bounds__(TT, 1) k_interp_tc(DevGrid G, EvalBatch b, con
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(B_DEMPTY + d));
-        // straight-line predicated stores, 8 columns per (uniform) step; a
-        // warp whose pixels all lie inside every member's window tests only
-        // the member count
+        // Straight-line stores, 8 columns per (uniform) step with their
+        // members read first; a warp whose pixels all lie inside every
+        // member's window tests only the member count, and not that in full
+        // steps.  (With a pointer read from the table before each store, the
+        // 64 shared-memory latencies in a row were 2,460 of a tile's 3,250
+        // cycles, and the products waited for the accumulators.)
         const int px = I.lo + i * TPX + 32 * q + lane;
-        if (__all_sync(0xffffffffu, px >= all_lo && px < all_hi)) {
+        char *base = reinterpret_cast<char *>(b.bufA + px);
+        const bool inside = __all_sync(0xffffffffu, px >= all_lo && px < all_hi);
 #pragma unroll
-          for (int c0 = 0; c0 < DCOLS; c0 += 8)
-            if (c0 < I.NP) {
+        for (int c0 = 0; c0 < DCOLS; c0 += 8)
+          if (c0 < I.NP) {
+            const uint4 ma = *reinterpret_cast<const uint4 *>(mem + c0), mb = *reinterpret_cast<const uint4 *>(mem + c0 + 4);
+            const unsigned mm[8] = {ma.x, ma.y, ma.z, ma.w, mb.x, mb.y, mb.z, mb.w};
+            if (inside && c0 + 8 <= I.nm) {
 #pragma unroll
-              for (int j = 0; j < 8; j++) st_if(rowp[c0 + j] + px, v[c0 + j], c0 + j < I.nm);
-            }
-        } else {
-#pragma unroll
-          for (int c0 = 0; c0 < DCOLS; c0 += 8)
-            if (c0 < I.NP) {
+              for (int j = 0; j < 8; j++) *reinterpret_cast<float *>(base + (size_t)mm[j] * row_bytes) = v[c0 + j];
+            } else {
 #pragma unroll
               for (int j = 0; j < 8; j++) {
                 const int n = c0 + j;
-                st_if(rowp[n] + px, v[n], n < I.nm && px >= wlo[n] && px < whi[n] && px < I.tc_hi);
+                st_if(reinterpret_cast<float *>(base + (size_t)mm[j] * row_bytes), v[n],
+                      n < I.nm && (inside || (px >= wlo[n] && px < whi[n] && px < I.tc_hi)));
               }
             }
-        }
+          }
       }
       // tail pixels [tail_start, hi): the reference's extra 1/65535 (interpolate.rs:978)
       if (!stop && I.hi > G.tail_start) {
@@ -504,15 +539,16 @@ __global__ void __launch_bounds__(TT, 1) k_interp_tc(DevGrid G, EvalBatch b, con
         for (int j = e; j < npx * I.nm; j += 32 * N_EP) {
           const int n = j / npx, px = t0 + j % npx;
           if (px < wlo[n] || px >= whi[n]) continue;
-          const EvalPrep &P = b.prep[I.R->member[n]];
+          const EvalPrep &P = b.prep[mem[n]];
           float acc = 0.0f;
+#pragma unroll 8
           for (int k = 0; k < 64; k++) {
+            // a missing row adds exactly 0: the sum is never -0
             const int col = I.R->col[k];
-            if (col < 0) continue;
-            const float x = (float)G.spectra[(size_t)col * G.stride + px];
-            acc = fmaf(P.w[k], __fmul_rn(__fdiv_rn(x, 65535.0f), I.R->f[k]), acc);
+            const float x = col >= 0 ? (float)G.spectra[(size_t)col * G.stride + px] : 0.0f;
+            acc = fmaf(col >= 0 ? P.w[k] : 0.0f, __fmul_rn(__fdiv_rn(x, 65535.0f), I.R->f[k]), acc);
           }
-          rowp[n][px] = acc;
+          b.bufA[(size_t)mem[n] * b.stride + px] = acc;
         }
       }
     }
