@@ -437,24 +437,23 @@ struct Workspace {
   DBuf<int> gcount;    // groups per segment
   DBuf<TcGroup> tcrec; // tensor-core interpolation groups, at each segment's first evaluation
   DBuf<int> tccount;   // tensor-core groups per segment
-  DBuf<int> tclist;    // indices of all tensor-core groups, and their count [1]
-  DBuf<int> tclist_count;
+  DBuf<int> tclist;    // indices of all tensor-core groups
+  DBuf<int> counters;  // CNT_* of kernels.h, zeroed together at the start of a batch
   DBuf<double> cpart;  // chunk chi2 partials [cap][MAX_CHUNKS]
-  DBuf<int> dlist;     // evaluations on the direct broadening path [cap], and their count [1]
+  DBuf<int> dlist;     // evaluations on the direct broadening path [cap]
   DBuf<double> zpart;  // tensor-core linear continua: partial coefficients [cap][LIN_MAX_SLICES][64]
-  DBuf<int> dcount;
   // merging of evaluations alone in their segment (EvalBatch::mkey)
   int mtab = 0;
-  DBuf<unsigned long long> mkey;
-  DBuf<int> mcnt, mmem, mslot, erec, mrcount;
+  DBuf<unsigned long long> mkey;  // [mtab] keys, then [mtab] int counts (zeroed together)
+  DBuf<int> mmem, mslot, erec;
   DBuf<GroupRec> mrec;
   void ensure(int64_t want, int64_t str, int bstr) {
     if (want <= cap && str == stride && bstr == bnd_stride) return;
     A.release(); B.release(); H.release(); HG.release(); prep.release();
     bnd.release(); cpart.release(); grec.release(); gcount.release();
-    tcrec.release(); tccount.release(); tclist.release(); tclist_count.release();
-    dlist.release(); dcount.release(); zpart.release();
-    mkey.release(); mcnt.release(); mmem.release(); mslot.release(); erec.release(); mrec.release(); mrcount.release();
+    tcrec.release(); tccount.release(); tclist.release(); counters.release();
+    dlist.release(); zpart.release();
+    mkey.release(); mmem.release(); mslot.release(); erec.release(); mrec.release();
     cap = 0;
     A.alloc((size_t)want * str);
     B.alloc((size_t)want * str);
@@ -467,19 +466,16 @@ struct Workspace {
     tcrec.alloc((size_t)want);
     tccount.alloc((size_t)want);
     tclist.alloc((size_t)want);
-    tclist_count.alloc(1);
+    counters.alloc(CNT_NUM);
     cpart.alloc((size_t)want * MAX_CHUNKS);
     dlist.alloc((size_t)want);
     zpart.alloc((size_t)want * LIN_MAX_SLICES * 64);
-    dcount.alloc(1);
     mtab = merge_table_slots(want);
-    mkey.alloc((size_t)mtab);
-    mcnt.alloc((size_t)mtab);
+    mkey.alloc((size_t)mtab * 3 / 2);
     mmem.alloc((size_t)mtab * MERGE_CAP);
-    mslot.alloc((size_t)mtab + 1);
+    mslot.alloc((size_t)mtab);
     erec.alloc((size_t)want);
     mrec.alloc((size_t)(want + 1) / 2);
-    mrcount.alloc(1);
     cap = want;
     stride = str;
     bnd_stride = bstr;
@@ -965,6 +961,7 @@ struct EvalArgs {
   uint32_t chunk_p1_mask = 0;    // chunk continua present, by coefficient count
   int max_chunks = 0;            // most chunks of those continua
   int other_cont = 0;            // linear / fixed / constant continua present
+  int late_resample = 0;         // a star k_broaden may leave to k_resample_obs (no instrument profile, or unsorted)
   int64_t max_nobs = 0;          // longest observed spectrum
   float *out_obs = nullptr;
   int64_t out_stride = 0;
@@ -987,6 +984,7 @@ void star_kinds(const std::vector<DevStar> &h, EvalArgs &a) {
     }
     a.max_nobs = std::max<int64_t>(a.max_nobs, st.n_obs);
     if (st.disp_kind != DISP_NONE) a.max_hg = std::max(a.max_hg, (st.gw - 1) / 2);
+    if (st.disp_kind == DISP_NONE || st.gw <= 1 || !st.obs_sorted) a.late_resample = 1;
     if (st.cont_kind == CONT_LINEAR && st.kp > 0) a.lin_kp_mask |= 1u << (st.kp / 16);
   }
 }
@@ -1075,6 +1073,7 @@ EvalBatch make_batch(pasta_grid *g, const EvalArgs &a, int64_t off, int64_t cnt)
   b.chunk_p1_mask = a.chunk_p1_mask;
   b.max_chunks = a.max_chunks;
   b.other_cont = a.other_cont;
+  b.late_resample = a.late_resample;
   // chi2 batches resample inside the broadening kernel unless a synth row is wanted
   b.obs_epi = a.need_chi2 && !a.out_obs && !a.out_synth && !a.full_window ? 1 : 0;
   b.bnd = g->ws.bnd.p;
@@ -1083,22 +1082,26 @@ EvalBatch make_batch(pasta_grid *g, const EvalArgs &a, int64_t off, int64_t cnt)
   // segments start at star boundaries; a sub-batch that starts inside a star
   // is cut in plain chunks of SEG
   b.seg_len = a.star_len > 0 && off % a.star_len == 0 ? a.star_len : 0;
-  const bool tc = interp_tc_enabled() && g->has_tmap;
+  // a segment shorter than the threshold has no tensor-core group
+  const int64_t longest = b.seg_len > 0 ? b.seg_len : cnt;
+  const bool tc = interp_tc_enabled() && g->has_tmap && std::min<int64_t>(longest, SEG) >= std::max(g->tc_min, TC_MIN_MEMBERS);
+  b.counters = g->ws.counters.p;
   b.tcrec = tc ? g->ws.tcrec.p : nullptr;
   b.tccount = g->ws.tccount.p;
   b.tclist = g->ws.tclist.p;
-  b.tclist_count = g->ws.tclist_count.p;
+  b.tclist_count = b.counters + CNT_TC;
   b.tmap = tc ? &g->tmap : nullptr;
   b.tc_min = g->tc_min;
-  if (interp_merge_enabled()) {
+  if (interp_merge_enabled() && num_segments(b) > 1) {  // one segment has nothing to merge with
     b.mkey = g->ws.mkey.p;
-    b.mcnt = g->ws.mcnt.p;
     b.mmem = g->ws.mmem.p;
     b.mslot = g->ws.mslot.p;
-    b.mtab = g->ws.mtab;
+    b.mtab = std::min(merge_table_slots(cnt), g->ws.mtab);
+    b.mcnt = reinterpret_cast<int *>(b.mkey + b.mtab);
     b.erec = g->ws.erec.p;
     b.mrec = g->ws.mrec.p;
-    b.mrcount = g->ws.mrcount.p;
+    b.mslot_count = b.counters + CNT_SLOTS;
+    b.mrcount = b.counters + CNT_MERGED;
   }
   b.bnd_stride = g->ws.bnd_stride;
   b.cpart = g->ws.cpart.p;
@@ -1107,7 +1110,7 @@ EvalBatch make_batch(pasta_grid *g, const EvalArgs &a, int64_t off, int64_t cnt)
   b.direct_max = g->direct_max;
   b.max_dtiles = (int)((g->npx + DIRECT_TILE - DIRECT_MAX_TAPS - 1) / (DIRECT_TILE - DIRECT_MAX_TAPS));
   b.direct_list = g->ws.dlist.p;
-  b.direct_count = g->ws.dcount.p;
+  b.direct_count = b.counters + CNT_DIRECT;
   // groups must start at star boundaries: sub-batches that begin inside a
   // group take the CUDA-core path
   const bool lin = linear_tc_enabled() && a.lin_group > 0 && a.lin_group <= 128 && off % a.lin_group == 0;
@@ -1742,7 +1745,7 @@ struct pasta_server {
   int max_m = 1, graph_max_m = 0;
   int64_t graph_gen = -1;
   uint32_t graph_mask = 0;  // continuum kinds / instrument width the captured step covers
-  int graph_other = 0, graph_hg = 0, graph_chunks = 0;
+  int graph_other = 0, graph_late = 0, graph_hg = 0, graph_chunks = 0;
   uint32_t graph_lin = 0;   // tensor-core linear bases the captured step covers
   cudaGraphExec_t exec = nullptr;
   cudaGraph_t graph = nullptr;
@@ -3675,6 +3678,7 @@ int pasta_server_step(pasta_server *sv) {
       star_kinds(occ, a);
       a.chunk_p1_mask |= sv->graph_mask;  // keep what the captured graph already covers
       if (sv->graph_other) a.other_cont = 1;
+      if (sv->graph_late) a.late_resample = 1;
       a.max_hg = std::max(a.max_hg, sv->graph_hg);
       a.max_chunks = std::max(a.max_chunks, sv->graph_chunks);
       a.lin_kp_mask |= sv->graph_lin;
@@ -3683,7 +3687,7 @@ int pasta_server_step(pasta_server *sv) {
     }
     ensure_workspace(g, E, a.max_nobs);
     const bool grown = sv->graph_max_m < sv->max_m || (a.chunk_p1_mask & ~sv->graph_mask) ||
-                       (a.other_cont && !sv->graph_other) || a.max_hg > sv->graph_hg ||
+                       (a.other_cont && !sv->graph_other) || (a.late_resample && !sv->graph_late) || a.max_hg > sv->graph_hg ||
                        a.max_chunks > sv->graph_chunks || (a.lin_kp_mask & ~sv->graph_lin);
     if (sv->exec && (grown || sv->graph_gen != g->ws.gen)) {
       // a wider kernel or a new continuum kind was admitted, or the workspace moved
@@ -3697,6 +3701,7 @@ int pasta_server_step(pasta_server *sv) {
       sv->graph_gen = g->ws.gen;
       sv->graph_mask = a.chunk_p1_mask;
       sv->graph_other = a.other_cont;
+      sv->graph_late = a.late_resample;
       sv->graph_hg = a.max_hg;
       sv->graph_chunks = a.max_chunks;
       sv->graph_lin = a.lin_kp_mask;

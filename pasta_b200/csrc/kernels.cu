@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(GROUP_T) k_group(DevGrid G, EvalBatch b) {
       }
       const int r = atomicAdd(&b.mcnt[slot], 1);
       if (r < MERGE_CAP) b.mmem[(size_t)slot * MERGE_CAP + r] = e;
-      if (r == 1) b.mslot[1 + atomicAdd(&b.mslot[0], 1)] = (int)slot;
+      if (r == 1) b.mslot[atomicAdd(b.mslot_count, 1)] = (int)slot;
       b.erec[e] = start + g;
     }
   }
@@ -269,9 +269,9 @@ constexpr int MERGE_W = 4;
 __global__ void __launch_bounds__(32 * MERGE_W) k_merge(DevGrid G, EvalBatch b) {
   __shared__ int mem[MERGE_W][MERGE_CAP + GROUP_MAX];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nlist = b.mslot[0];
+  const int nlist = *b.mslot_count;
   for (int j = blockIdx.x * MERGE_W + warp; j < nlist; j += gridDim.x * MERGE_W) {
-    const int slot = b.mslot[1 + j], nc = min(b.mcnt[slot], MERGE_CAP);
+    const int slot = b.mslot[j], nc = min(b.mcnt[slot], MERGE_CAP);
     const int *list = b.mmem + (size_t)slot * MERGE_CAP;
     const int e0 = list[0];
     int nt = 0;  // the matching evaluations, in list order
@@ -298,13 +298,7 @@ __global__ void __launch_bounds__(32 * MERGE_W) k_merge(DevGrid G, EvalBatch b) 
 
 void launch_group(const DevGrid &G, const EvalBatch &b, cudaStream_t s) {
   if (b.E <= 0) return;
-  if (b.tcrec) cudaMemsetAsync(b.tclist_count, 0, sizeof(int), s);
-  if (b.mkey) {
-    cudaMemsetAsync(b.mkey, 0, (size_t)b.mtab * sizeof(unsigned long long), s);
-    cudaMemsetAsync(b.mcnt, 0, (size_t)b.mtab * sizeof(int), s);
-    cudaMemsetAsync(b.mslot, 0, sizeof(int), s);
-    cudaMemsetAsync(b.mrcount, 0, sizeof(int), s);
-  }
+  if (b.mkey) cudaMemsetAsync(b.mkey, 0, (size_t)b.mtab * (sizeof(unsigned long long) + sizeof(int)), s);  // and mcnt
   k_group<<<num_segments(b), GROUP_T, 0, s>>>(G, b);
   count_launch();
   if (b.mkey) {
@@ -1142,7 +1136,9 @@ void launch_pipeline(const DevGrid &G, const EvalBatch &b, const float2 *tw, con
     launch_gauss(G, b, s);
   }
   if (b.need_chi2) {
-    launch_resample_obs(G, b, s);
+    // k_broaden resamples every evaluation with an instrument profile and
+    // sorted pixels, unless another kernel broadens it
+    if (b.late_resample || b.direct_max > 0 || o.may_unfuse || !b.obs_epi) launch_resample_obs(G, b, s);
     launch_chi2(G, b, s);
   } else if (b.status) {
     launch_prep_status(b, s);

@@ -38,6 +38,9 @@ struct __align__(16) TcGroup {
   int pad;
 };
 
+// EvalBatch::counters: tensor-core groups, direct evaluations, merge slots, merged records
+enum { CNT_TC = 0, CNT_DIRECT, CNT_SLOTS, CNT_MERGED, CNT_NUM };
+
 constexpr int LIN_MAX_SLICES = 32;  // at most MAX_CHUNKS: the slices' residual sums use EvalBatch::cpart
 
 // Per-launch description of one batch of evaluations.
@@ -61,6 +64,7 @@ struct EvalBatch {
   int need_chi2;
   uint32_t chunk_p1_mask;    // bit p1 set: a chunk continuum with p1 coefficients is present
   int other_cont;            // a linear / fixed / constant continuum is present
+  int late_resample;         // k_broaden may leave some star's evaluations to k_resample_obs
   int max_chunks;            // most chunks of any chunk continuum in the batch
   int obs_epi;               // chi2 batches: resample inside k_broaden, synth rows are not kept
   int *bnd;                  // [E][bnd_stride] first observed pixel of every broadening block
@@ -71,11 +75,12 @@ struct EvalBatch {
   // first evaluation, so a star's groups do not depend on the rest of the
   // batch.  A segment's records sit at its first evaluation's index.
   int seg_len;
+  int *counters;             // [CNT_NUM] the counts below, zeroed before k_prep (null: none used)
   GroupRec *grec;            // [E] groups of each segment, in order
   int *gcount;               // [segments] groups per segment
   TcGroup *tcrec;            // [E] tensor-core groups of each segment (null: none)
   int *tclist;               // [E] indices into tcrec of all tensor-core groups, in any order
-  int *tclist_count;         // [1] their number (zeroed before k_group)
+  int *tclist_count;         // [1] their number
   int tc_min;                // members a tensor-core group needs (TC_MIN_MEMBERS .. SEG; larger: none)
   int *tccount;              // [segments]
   // Evaluations that end up alone in their segment (spread swarms: the early
@@ -83,10 +88,10 @@ struct EvalBatch {
   // have the same neighbour columns, in groups of up to GROUP_MAX, when mkey
   // is set (null: off).  Merging changes no result: every member keeps its
   // own accumulators and row order.
-  unsigned long long *mkey;  // [mtab] hash of the columns per table slot (0: empty); zeroed before k_group
-  int *mcnt;                 // [mtab] evaluations that chose each slot; zeroed before k_group
+  unsigned long long *mkey;  // [mtab] EvalPrep::key per table slot (0: empty); zeroed before k_group
+  int *mcnt;                 // [mtab] evaluations that chose each slot, right after mkey (zeroed with it)
   int *mmem;                 // [mtab][MERGE_CAP] the first MERGE_CAP of them
-  int *mslot;                // [1 + mtab] number of slots with two or more evaluations, then the slots
+  int *mslot, *mslot_count;  // slots with two or more evaluations, and their number [1]
   int mtab;                  // table slots (a power of two, at least 2 E)
   int *erec;                 // [E] record index of the evaluation's own (alone) group
   GroupRec *mrec;            // [(E + 1) / 2] merged group records (at most half the evaluations)
@@ -97,7 +102,7 @@ struct EvalBatch {
   int direct_max;            // combined kernels of at most this many taps are convolved directly (0: never)
   int max_dtiles;            // direct tiles per evaluation at most (at least DIRECT_TILE - DIRECT_MAX_TAPS outputs each)
   int *direct_list;          // [E] evaluations k_prep routed to the direct path (in any order)
-  int *direct_count;         // [1] their number (zeroed before k_prep)
+  int *direct_count;         // [1] their number
   int lin_group;             // linear continua on the tensor cores: groups of this many consecutive
                              // evaluations share a star (0: the CUDA-core path)
   uint32_t lin_kp_mask;      // bit kp / 16: a linear continuum with a kp-column tensor-core basis is present

@@ -249,6 +249,7 @@ extern "C" int pasta_chi2_noalloc(const pasta_grid *g, const pasta_dispersion *d
   b.max_chunks = star.cont_kind == CONT_CHUNK ? star.n_chunks : 0;
   b.other_cont = star.cont_kind == CONT_CHUNK ? 0 : 1;
   b.obs_epi = 1;
+  b.late_resample = 1;
   b.bnd = bnd;
   b.bnd_stride = bstr;
   b.cpart = cpart;

@@ -293,13 +293,13 @@ __global__ void __launch_bounds__(FFT_T) k_rotker(DevGrid G, EvalBatch b, const 
 
 void launch_prep(const DevGrid &G, const EvalBatch &b, cudaStream_t s) {
   if (b.E <= 0) return;
-  if (b.direct_max > 0 && b.direct_count) cudaMemsetAsync(b.direct_count, 0, sizeof(int), s);
+  if (b.counters) cudaMemsetAsync(b.counters, 0, CNT_NUM * sizeof(int), s);
   k_prep<<<(b.E + PREP_T / PREP_L - 1) / (PREP_T / PREP_L), PREP_T, 0, s>>>(G, b, 0);
   count_launch();
 }
 void launch_prep_full(const DevGrid &G, const EvalBatch &b, cudaStream_t s) {
   if (b.E <= 0) return;
-  if (b.direct_max > 0 && b.direct_count) cudaMemsetAsync(b.direct_count, 0, sizeof(int), s);
+  if (b.counters) cudaMemsetAsync(b.counters, 0, CNT_NUM * sizeof(int), s);
   k_prep<<<(b.E + PREP_T / PREP_L - 1) / (PREP_T / PREP_L), PREP_T, 0, s>>>(G, b, 1);
   count_launch();
 }

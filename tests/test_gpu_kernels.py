@@ -193,3 +193,30 @@ def test_calls_from_several_threads(env):
     for t in threads:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize("kind", ["none", "unsorted"])
+@pytest.mark.parametrize("n", [1, 70])
+def test_evaluations_resampled_after_the_broadening(env, kind, n):
+    """Stars whose evaluations k_broaden leaves to the later resampling (no instrument profile with vsini 0 among the
+    labels, or unsorted pixels), in one segment and in two, against the oracle in double."""
+    import oracle as O
+    P, S, spec, interp, star = env["P"], env["S"], env["spec"], env["interp"], env["star"]
+    order = np.arange(len(star.wl))
+    if kind == "unsorted":
+        order = np.random.default_rng(4).permutation(len(order))
+    wl, flux, var = star.wl[order], star.flux[order], star.var[order]
+    ones = np.ones(len(wl), np.float32)
+    lab = _near(star, n, 77)
+    lab[::3, 3] = 0.0
+    labels, spectra, factors = S.make_grid(spec)
+    og = O.Grid(labels, spectra, factors, O.WL_LOGSPACE, spec.log_first, spec.log_step)
+    if kind == "none":
+        disp, od = P.NoConvolutionDispersion(wl, env["wl"]), O.Disp(og, O.DISP_NONE, wl)
+    else:
+        disp, od = P.FixedResolutionDispersion(wl, 85000.0, env["wl"]), O.Disp(og, O.DISP_FIXED, wl, 85000.0)
+    fitter = interp.get_fitter(disp, P.FixedContinuum(ones), P.PSOSettings(8, 2), (0.0, 300.0), (-150.0, 150.0))
+    got = np.array(fitter.chi2(interp, flux, var, lab))
+    ref, st = O.chi2(og, od, O.Cont(O.CONT_FIXED, continuum=ones), flux, var, lab, O.F64)
+    assert (st == 0).all()
+    np.testing.assert_allclose(got, ref, rtol=CHI2_TOL)
