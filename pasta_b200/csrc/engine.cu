@@ -214,6 +214,8 @@ struct Stage {
 struct Ctx {
   int dev = 0;
   cudaStream_t stream = nullptr;
+  cudaStream_t side = nullptr;                  // see PipelineOpts::side
+  cudaEvent_t fork = nullptr, join = nullptr;
   DBuf<float2> tw;  // W_2048^k
   Stage stage;
   std::mutex scratch_mu;
@@ -238,6 +240,9 @@ Ctx &ctx() {
     c->dev = g_dev;
     CK(cudaSetDevice(g_dev));
     CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
+    CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming));
     std::vector<float2> t(FFTN);
     for (int k = 0; k < FFTN; k++) {
       double a = -2.0 * M_PI * (double)k / (double)FFTN;
@@ -1131,6 +1136,9 @@ void run_evals(pasta_grid *g, const EvalArgs &a, cudaStream_t s) {
   o.full_window = a.full_window;
   o.rot = a.max_m > 1;
   o.may_unfuse = may_unfuse;
+  o.side = C.side;
+  o.fork = C.fork;
+  o.join = C.join;
   for (int64_t off = 0; off < a.E; off += cap) {
     const int64_t cnt = std::min(cap, a.E - off);
     EvalBatch b = make_batch(g, a, off, cnt);

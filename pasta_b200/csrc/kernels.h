@@ -118,6 +118,10 @@ struct PipelineOpts {
   int full_window = 0;       // every synthetic pixel, no resampling (interpolate entry points)
   int rot = 1;               // some evaluation may rotate (launch the rotation spectra)
   int may_unfuse = 0;        // some evaluation may need the unfused path
+  // a second stream and two events: the rotation spectra and block bounds run
+  // beside the grouping and interpolation (null: all on the one stream)
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
 };
 void launch_pipeline(const DevGrid &G, const EvalBatch &b, const float2 *twiddle, const PipelineOpts &o,
                      cudaStream_t s);
