@@ -201,8 +201,9 @@ struct GraphHold {
 };
 
 // Page-locked staging for the copies of host arrays: pageable copies run at
-// 6-8 GB/s and wait (61 models of 37,501 pixels, 9 MB: 1.5 -> 1.1 ms).  Two halves in turn; a half is written again once the
-// copy that used it is done (its event).
+// 6-8 GB/s and wait (61 models of 37,501 pixels, 9 MB: 1.5 -> 1.1 ms).  Two
+// halves in turn; a half is written again once the copy that used it is done
+// (its event).
 constexpr size_t STAGE_HALF = 4ull << 20, STAGE_MIN = 64ull << 10;
 struct Stage {
   std::mutex mu;

@@ -220,3 +220,25 @@ def test_evaluations_resampled_after_the_broadening(env, kind, n):
     ref, st = O.chi2(og, od, O.Cont(O.CONT_FIXED, continuum=ones), flux, var, lab, O.F64)
     assert (st == 0).all()
     np.testing.assert_allclose(got, ref, rtol=CHI2_TOL)
+
+
+@pytest.mark.parametrize("resolution", [20000.0, 40000.0, 60000.0, 85000.0, 200000.0])
+@pytest.mark.parametrize("vsini,rv", [(0.0, 0.0), (60.0, 0.0), (299.0, 20.0)])
+def test_per_pixel_instrument_kernels(env, resolution, vsini, rv):
+    """Per-pixel instrument kernels of several widths in the broadening blocks, over the whole grid (both ends pass
+    through, the last block stands alone or half empty), against the oracle in single precision (1e-5 of the maximum)."""
+    import oracle as O
+    P, S, spec, interp = env["P"], env["S"], env["spec"], env["interp"]
+    wl = spec.wl()[:-1] if rv == 0.0 else np.geomspace(spec.wl()[0] * 1.001, spec.wl()[-2] * 0.999, 3001)
+    sig = (wl / (resolution * np.linspace(1.0, 1.5, len(wl))) / 2.355).astype(np.float32)
+    labels, spectra, factors = S.make_grid(spec)
+    og = O.Grid(labels, spectra, factors, O.WL_LOGSPACE, spec.log_first, spec.log_step)
+    lab = [7130.0, 0.07, 4.02, vsini, rv]
+    keep = interp.direct_max
+    try:
+        interp.direct_max = 0  # the FFT path
+        got = interp.produce_model(P.VariableResolutionDispersion(wl, sig, env["wl"]), *lab)
+    finally:
+        interp.direct_max = keep
+    ref = O.Disp(og, O.DISP_VARIABLE, wl, disp=sig).produce_model(lab, O.F32)
+    assert np.abs(got.astype(np.float64) - ref).max() <= 1e-5 * np.abs(ref).max()
