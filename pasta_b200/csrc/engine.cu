@@ -15,7 +15,6 @@
 #include <limits>
 #include <chrono>
 #include <cmath>
-#include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -23,8 +22,6 @@
 #include <map>
 #include <memory>
 #include <mutex>
-#include <system_error>
-#include <thread>
 #include <stdexcept>
 #include <string>
 #include <array>
@@ -32,6 +29,7 @@
 
 #include "../../include/pasta_b200.h"
 #include "common.cuh"
+#include "hostmem.h"
 #include "kernels.h"
 
 using namespace pb;
@@ -39,24 +37,6 @@ using namespace pb;
 namespace {
 
 thread_local std::string g_last_error;
-
-struct PErr : std::runtime_error {
-  int code;
-  PErr(int c, const std::string &m) : std::runtime_error(m), code(c) {}
-};
-[[noreturn]] void fail(int code, const char *fmt, ...) {
-  char buf[1024];
-  va_list ap;
-  va_start(ap, fmt);
-  vsnprintf(buf, sizeof buf, fmt, ap);
-  va_end(ap);
-  throw PErr(code, buf);
-}
-#define CK(call)                                                                                 \
-  do {                                                                                           \
-    cudaError_t e_ = (call);                                                                     \
-    if (e_ != cudaSuccess) fail(PASTA_E_CUDA, "%s failed: %s", #call, cudaGetErrorString(e_)); \
-  } while (0)
 
 template <class F>
 int guard(F &&f) {
@@ -91,330 +71,6 @@ const char *status_message(int s) {
     default: return "error";
   }
 }
-
-// ---------------------------------------------------------------- memory
-// Scratch memory of the entry points, kept per device between calls: a call
-// allocated and freed 8 to 30 buffers, and each cudaFree waits for the device
-// (with the staging below: one model of 15,000 pixels 161 -> 125 us, chi2 of 40
-// labels 239 -> 182 us, of 160 binary labels 1.30 -> 0.59 ms end to end, and a
-// batch of fits no longer varies between 28 and 158 ms).
-// Bounded (SCRATCH_BLOCK per block, SCRATCH_TOTAL in all; anything larger goes
-// straight to cudaMalloc and cudaFree), given back when a grid is destroyed or
-// an allocation fails.  A block may still be read by work in flight when it is
-// put back (that work is on the device's one stream): the first block taken
-// after any was put back waits for the stream.
-constexpr size_t SCRATCH_BLOCK = 64ull << 20, SCRATCH_TOTAL = 256ull << 20;
-void *scratch_take(size_t bytes, size_t *got);
-void scratch_put(void *p, size_t bytes, int dev);
-int scratch_device();
-cudaStream_t scratch_stream();
-void scratch_flush(int dev);
-
-// POOL: scratch of one call or fit (see scratch_take); its uploads are ordered
-// on the device's stream
-template <class T, bool POOL = false>
-struct DBuf {
-  T *p = nullptr;
-  size_t n = 0;
-  size_t bytes = 0;  // of the scratch block
-  int dev = -1;
-  DBuf() = default;
-  DBuf(const DBuf &) = delete;
-  DBuf &operator=(const DBuf &) = delete;
-  ~DBuf() { release(); }
-  void release() {
-    if (p) {
-      if (POOL) scratch_put(p, bytes, dev);
-      else cudaFree(p);
-    }
-    p = nullptr;
-    n = 0;
-  }
-  void alloc(size_t count) {
-    release();
-    if (count == 0) return;
-    if (POOL) {
-      dev = scratch_device();
-      p = (T *)scratch_take(count * sizeof(T), &bytes);
-    } else {
-      cudaError_t e = cudaMalloc(&p, count * sizeof(T));
-      if (e != cudaSuccess) {
-        p = nullptr;
-        cudaGetLastError();
-        scratch_flush(-1);
-        e = cudaMalloc(&p, count * sizeof(T));
-      }
-      if (e != cudaSuccess) {
-        p = nullptr;
-        cudaGetLastError();
-        fail(PASTA_E_NOMEM, "cudaMalloc of %zu bytes failed: %s", count * sizeof(T), cudaGetErrorString(e));
-      }
-    }
-    n = count;
-  }
-  void upload(const T *h, size_t count) {
-    alloc(count);
-    if (!count) return;
-    if (POOL) CK(cudaMemcpyAsync(p, h, count * sizeof(T), cudaMemcpyHostToDevice, scratch_stream()));
-    else CK(cudaMemcpy(p, h, count * sizeof(T), cudaMemcpyHostToDevice));
-  }
-  void upload(const std::vector<T> &v) { upload(v.data(), v.size()); }
-};
-template <class T>
-using SBuf = DBuf<T, true>;
-
-// page-locked host buffer: copies from and to it are asynchronous and can
-// be captured in a CUDA graph
-template <class T>
-struct HostBuf {
-  T *p = nullptr;
-  HostBuf() = default;
-  HostBuf(const HostBuf &) = delete;
-  HostBuf &operator=(const HostBuf &) = delete;
-  ~HostBuf() {
-    if (p) cudaFreeHost(p);
-  }
-  void alloc(size_t count) {
-    if (p) cudaFreeHost(p);
-    p = nullptr;
-    if (count == 0) return;
-    cudaError_t e = cudaMallocHost(&p, count * sizeof(T));
-    if (e != cudaSuccess) {
-      p = nullptr;
-      cudaGetLastError();
-      fail(PASTA_E_NOMEM, "cudaMallocHost of %zu bytes failed: %s", count * sizeof(T), cudaGetErrorString(e));
-    }
-  }
-};
-
-// an instantiated CUDA graph, destroyed with its owner
-struct GraphHold {
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  GraphHold() = default;
-  GraphHold(const GraphHold &) = delete;
-  GraphHold &operator=(const GraphHold &) = delete;
-  ~GraphHold() {
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
-  }
-};
-
-// Page-locked staging for the copies of host arrays: pageable copies run at
-// 6-8 GB/s and wait (61 models of 37,501 pixels, 9 MB: 1.5 -> 1.1 ms).  Two
-// halves in turn; a half is written again once the copy that used it is done
-// (its event).
-constexpr size_t STAGE_HALF = 4ull << 20, STAGE_MIN = 64ull << 10;
-struct Stage {
-  std::mutex mu;
-  HostBuf<unsigned char> buf;
-  cudaEvent_t ev[2] = {};
-  int at = 0;       // half in use
-  size_t fill = 0;  // bytes used of it
-};
-struct Ctx {
-  int dev = 0;
-  cudaStream_t stream = nullptr;
-  cudaStream_t side = nullptr;                  // see PipelineOpts::side
-  cudaEvent_t fork = nullptr, join = nullptr;
-  DBuf<float2> tw;  // W_2048^k
-  Stage stage;
-  std::mutex scratch_mu;
-  std::multimap<size_t, void *> scratch;  // free blocks by size
-  size_t scratch_total = 0;
-  bool scratch_dirty = false;  // blocks were put back since the last wait for the stream
-};
-std::mutex g_ctx_mu;
-std::map<int, std::unique_ptr<Ctx>> g_ctx;
-thread_local int g_dev = -1;
-
-Ctx &ctx() {
-  if (g_dev < 0) {
-    int d;
-    CK(cudaGetDevice(&d));
-    g_dev = d;
-  }
-  std::lock_guard<std::mutex> lk(g_ctx_mu);
-  auto &c = g_ctx[g_dev];
-  if (!c) {
-    c.reset(new Ctx());
-    c->dev = g_dev;
-    CK(cudaSetDevice(g_dev));
-    CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-    CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
-    CK(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming));
-    std::vector<float2> t(FFTN);
-    for (int k = 0; k < FFTN; k++) {
-      double a = -2.0 * M_PI * (double)k / (double)FFTN;
-      t[k] = make_float2((float)std::cos(a), (float)std::sin(a));
-    }
-    c->tw.upload(t);
-  }
-  CK(cudaSetDevice(c->dev));
-  return *c;
-}
-
-// ------------------------------------------------------------ scratch pool
-int scratch_device() { return ctx().dev; }
-cudaStream_t scratch_stream() { return ctx().stream; }
-size_t scratch_round(size_t b) {  // 512 bytes, or an eighth of the power of two below
-  size_t step = 512;
-  while (step * 16 <= b) step *= 2;
-  return (b + step - 1) / step * step;
-}
-void scratch_flush(int dev) {
-  std::unique_lock<std::mutex> lk(g_ctx_mu, std::try_to_lock);
-  if (!lk.owns_lock()) return;  // a context is being made: nothing is cached for it yet
-  for (auto &kv : g_ctx) {
-    if (dev >= 0 && kv.first != dev) continue;
-    Ctx &C = *kv.second;
-    std::lock_guard<std::mutex> l2(C.scratch_mu);
-    for (auto &b : C.scratch) cudaFree(b.second);  // waits for the device
-    C.scratch.clear();
-    C.scratch_total = 0;
-    C.scratch_dirty = false;
-  }
-}
-void *scratch_take(size_t bytes, size_t *got) {
-  Ctx &C = ctx();
-  const size_t want = scratch_round(bytes);
-  *got = want;
-  if (want <= SCRATCH_BLOCK) {
-    std::lock_guard<std::mutex> lk(C.scratch_mu);
-    auto it = C.scratch.lower_bound(want);
-    if (it != C.scratch.end() && it->first <= 2 * want + (64u << 10)) {
-      if (C.scratch_dirty) {
-        CK(cudaStreamSynchronize(C.stream));
-        C.scratch_dirty = false;
-      }
-      void *p = it->second;
-      *got = it->first;
-      C.scratch_total -= it->first;
-      C.scratch.erase(it);
-      return p;
-    }
-  }
-  void *p = nullptr;
-  cudaError_t e = cudaMalloc(&p, want);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    scratch_flush(-1);
-    e = cudaMalloc(&p, want);
-  }
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    fail(PASTA_E_NOMEM, "cudaMalloc of %zu bytes failed: %s", want, cudaGetErrorString(e));
-  }
-  return p;
-}
-void scratch_put(void *p, size_t bytes, int dev) {
-  Ctx *C = nullptr;
-  {
-    std::lock_guard<std::mutex> lk(g_ctx_mu);
-    auto it = g_ctx.find(dev);
-    if (it != g_ctx.end()) C = it->second.get();
-  }
-  if (C && bytes <= SCRATCH_BLOCK) {
-    std::lock_guard<std::mutex> lk(C->scratch_mu);
-    if (C->scratch_total + bytes <= SCRATCH_TOTAL) {
-      C->scratch.emplace(bytes, p);
-      C->scratch_total += bytes;
-      C->scratch_dirty = true;
-      return;
-    }
-  }
-  cudaFree(p);
-}
-
-// ------------------------------------------------------------- host copies
-// memcpy of large arrays by a few threads (one core moves 8-10 GB/s, less
-// into pages touched for the first time)
-void copy_threads(void *dst, const void *src, size_t n) {
-  const size_t parts = std::min<size_t>(4, n >> 20);
-  if (parts < 2) {
-    std::memcpy(dst, src, n);
-    return;
-  }
-  std::vector<std::thread> th;
-  const size_t per = (n / parts + 4095) & ~(size_t)4095;
-  for (size_t k = 1; k < parts; k++) {
-    const size_t o = k * per, m = k + 1 == parts ? n - o : per;
-    try {
-      th.emplace_back([=] { std::memcpy((char *)dst + o, (const char *)src + o, m); });
-    } catch (const std::system_error &) {  // no thread to be had
-      std::memcpy((char *)dst + o, (const char *)src + o, m);
-    }
-  }
-  std::memcpy(dst, src, per);
-  for (auto &t : th) t.join();
-}
-
-// Copies between host arrays and the device through the staging buffer, in
-// order on the device's stream; pageable copies while another thread holds it.
-struct HostCopy {
-  Ctx &C;
-  std::unique_lock<std::mutex> lk;
-  bool ok;
-  explicit HostCopy(Ctx &c) : C(c), lk(c.stage.mu, std::try_to_lock), ok(lk.owns_lock()) {
-    Stage &S = C.stage;
-    if (ok && !S.buf.p) {
-      S.buf.alloc(2 * STAGE_HALF);
-      for (auto &e : S.ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    }
-  }
-  // room for n bytes (at most STAGE_HALF) in the current half, or the next one
-  unsigned char *room(size_t n) {
-    Stage &S = C.stage;
-    if (S.fill + n > STAGE_HALF) {
-      CK(cudaEventRecord(S.ev[S.at], C.stream));
-      S.at ^= 1;
-      S.fill = 0;
-      CK(cudaEventSynchronize(S.ev[S.at]));
-    }
-    unsigned char *p = S.buf.p + (size_t)S.at * STAGE_HALF + S.fill;
-    S.fill += (n + 255) & ~(size_t)255;
-    return p;
-  }
-  void up(void *dst, const void *src, size_t n) {
-    if (!ok) {
-      CK(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, C.stream));
-      return;
-    }
-    for (size_t o = 0; o < n;) {
-      const size_t m = std::min(n - o, STAGE_HALF);
-      unsigned char *p = room(m);
-      copy_threads(p, (const char *)src + o, m);
-      CK(cudaMemcpyAsync((char *)dst + o, p, m, cudaMemcpyHostToDevice, C.stream));
-      o += m;
-    }
-  }
-  // waits for the copy; the next part is on its way while one is copied out
-  void down(void *dst, const void *src, size_t n) {
-    if (!ok || n < STAGE_MIN) {
-      CK(cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToHost, C.stream));
-      CK(cudaStreamSynchronize(C.stream));
-      return;
-    }
-    Stage &S = C.stage;
-    CK(cudaStreamSynchronize(C.stream));  // both halves free
-    S.at = 0;
-    S.fill = STAGE_HALF;  // the next upload starts on the other half
-    const size_t parts = (n + STAGE_HALF - 1) / STAGE_HALF;
-    auto issue = [&](size_t k) {
-      const size_t o = k * STAGE_HALF, m = std::min(n - o, STAGE_HALF);
-      CK(cudaMemcpyAsync(S.buf.p + (k & 1) * STAGE_HALF, (const char *)src + o, m, cudaMemcpyDeviceToHost, C.stream));
-      CK(cudaEventRecord(S.ev[k & 1], C.stream));
-    };
-    issue(0);
-    for (size_t k = 0; k < parts; k++) {
-      if (k + 1 < parts) issue(k + 1);
-      CK(cudaEventSynchronize(S.ev[k & 1]));
-      const size_t o = k * STAGE_HALF, m = std::min(n - o, STAGE_HALF);
-      copy_threads((char *)dst + o, S.buf.p + (k & 1) * STAGE_HALF, m);
-    }
-  }
-};
 
 double now_s() {
   return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
