@@ -82,7 +82,9 @@ struct DBuf {
     p = nullptr;
     n = 0;
   }
-  void alloc(size_t count) {
+  // flush: give the scratch pools back and try again when there is no memory
+  // (not under g_ctx_mu, which the flush takes)
+  void alloc(size_t count, bool flush = true) {
     release();
     if (count == 0) return;
     if (POOL) {
@@ -93,8 +95,10 @@ struct DBuf {
       if (e != cudaSuccess) {
         p = nullptr;
         cudaGetLastError();
-        scratch_flush(-1);
-        e = cudaMalloc(&p, count * sizeof(T));
+        if (flush) {
+          scratch_flush(-1);
+          e = cudaMalloc(&p, count * sizeof(T));
+        }
       }
       if (e != cudaSuccess) {
         p = nullptr;
@@ -201,7 +205,8 @@ Ctx &ctx() {
       double a = -2.0 * M_PI * (double)k / (double)FFTN;
       t[k] = make_float2((float)std::cos(a), (float)std::sin(a));
     }
-    c->tw.upload(t);
+    c->tw.alloc(t.size(), false);
+    CK(cudaMemcpy(c->tw.p, t.data(), t.size() * sizeof(float2), cudaMemcpyHostToDevice));
   }
   CK(cudaSetDevice(c->dev));
   return *c;
@@ -216,8 +221,7 @@ size_t scratch_round(size_t b) {  // 512 bytes, or an eighth of the power of two
   return (b + step - 1) / step * step;
 }
 void scratch_flush(int dev) {
-  std::unique_lock<std::mutex> lk(g_ctx_mu, std::try_to_lock);
-  if (!lk.owns_lock()) return;  // a context is being made: nothing is cached for it yet
+  std::lock_guard<std::mutex> lk(g_ctx_mu);
   for (auto &kv : g_ctx) {
     if (dev >= 0 && kv.first != dev) continue;
     Ctx &C = *kv.second;

@@ -1,0 +1,167 @@
+// Failure paths of pasta_b200/csrc/hostmem.h on the CPU: the CUDA runtime is
+// replaced by the stand-ins below, whose calls can be made to fail.
+//   hostmem_cases <case>     exit code 0: passed
+#include <atomic>
+#include <chrono>
+#include <cstdlib>
+#include <cstring>
+#include <new>
+#include <set>
+
+#include "../pasta_b200/csrc/hostmem.h"
+
+// ------------------------------------------------- a runtime that can fail
+namespace fake {
+std::mutex mu;
+size_t capacity = 1ull << 40, used = 0;  // "device memory" (nothing that large is touched)
+std::map<void *, size_t> blocks;
+std::vector<size_t> asked;               // sizes of all device allocations, in order
+std::atomic<bool> pinned_fails{false}, events_fail{false}, streams_fail{false};
+std::atomic<uintptr_t> next_handle{16};
+std::set<cudaEvent_t> events;
+cudaError_t last = cudaSuccess;
+cudaError_t set(cudaError_t e) {
+  if (e != cudaSuccess) last = e;
+  return e;
+}
+}  // namespace fake
+
+extern "C" {
+cudaError_t cudaMalloc(void **p, size_t n) {
+  std::lock_guard<std::mutex> lk(fake::mu);
+  fake::asked.push_back(n);
+  if (fake::used + n > fake::capacity) {
+    *p = nullptr;
+    return fake::set(cudaErrorMemoryAllocation);
+  }
+  *p = std::malloc(std::min<size_t>(n, 64u << 20));
+  fake::blocks[*p] = n;
+  fake::used += n;
+  return cudaSuccess;
+}
+cudaError_t cudaFree(void *p) {
+  std::lock_guard<std::mutex> lk(fake::mu);
+  auto it = fake::blocks.find(p);
+  if (it == fake::blocks.end()) return fake::set(cudaErrorInvalidValue);
+  fake::used -= it->second;
+  fake::blocks.erase(it);
+  std::free(p);
+  return cudaSuccess;
+}
+cudaError_t cudaMallocHost(void **p, size_t n) {
+  if (fake::pinned_fails) return fake::set(cudaErrorMemoryAllocation);
+  *p = std::malloc(n);
+  return cudaSuccess;
+}
+cudaError_t cudaFreeHost(void *p) {
+  std::free(p);
+  return cudaSuccess;
+}
+cudaError_t cudaGetLastError(void) {
+  const cudaError_t e = fake::last;
+  fake::last = cudaSuccess;
+  return e;
+}
+const char *cudaGetErrorString(cudaError_t) { return "stand-in error"; }
+cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) {
+  std::memcpy(d, s, n);
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t st) {
+  if (!st) return fake::set(cudaErrorInvalidResourceHandle);
+  std::memcpy(d, s, n);
+  return cudaSuccess;
+}
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
+  if (fake::streams_fail) return fake::set(cudaErrorMemoryAllocation);
+  *s = (cudaStream_t)(fake::next_handle += 16);
+  return cudaSuccess;
+}
+cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
+  if (fake::events_fail) return fake::set(cudaErrorMemoryAllocation);
+  *e = (cudaEvent_t)(fake::next_handle += 16);
+  std::lock_guard<std::mutex> lk(fake::mu);
+  fake::events.insert(*e);
+  return cudaSuccess;
+}
+cudaError_t cudaEventDestroy(cudaEvent_t e) {
+  std::lock_guard<std::mutex> lk(fake::mu);
+  return fake::events.erase(e) ? cudaSuccess : fake::set(cudaErrorInvalidResourceHandle);
+}
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) {
+  std::lock_guard<std::mutex> lk(fake::mu);
+  return fake::events.count(e) ? cudaSuccess : fake::set(cudaErrorInvalidResourceHandle);
+}
+cudaError_t cudaEventSynchronize(cudaEvent_t e) { return cudaEventRecord(e, nullptr); }
+cudaError_t cudaGetDevice(int *d) {
+  *d = 0;
+  return cudaSuccess;
+}
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
+cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
+}
+
+#define EXPECT(cond)                                                     \
+  do {                                                                   \
+    if (!(cond)) {                                                       \
+      std::fprintf(stderr, "%s:%d: %s\n", __FILE__, __LINE__, #cond);    \
+      std::_Exit(1);                                                     \
+    }                                                                    \
+  } while (0)
+
+// ------------------------------------------------------------------- cases
+// An allocation that only fits once the pool's free blocks are given back
+// succeeds, also while another thread is inside ctx() or a release.
+static void flush_while_contexts_are_looked_up() {
+  ctx();
+  {
+    SBuf<char> a, b, c;
+    a.alloc(60u << 20);
+    b.alloc(60u << 20);
+    c.alloc(60u << 20);
+  }
+  EXPECT(ctx().scratch_total >= (180u << 20));
+  fake::capacity = 300ull << 20;
+  std::atomic<bool> held{false};
+  std::thread other([&] {
+    std::lock_guard<std::mutex> lk(g_ctx_mu);
+    held = true;
+    std::this_thread::sleep_for(std::chrono::milliseconds(200));
+  });
+  while (!held) std::this_thread::yield();
+  DBuf<char> big;
+  int code = 0;
+  try {
+    // past the context lookup a scratch buffer makes: straight to the allocation
+    big.alloc(200u << 20);
+  } catch (const PErr &e) {
+    code = e.code;
+  }
+  other.join();
+  EXPECT(code == 0 && big.p);
+  EXPECT(ctx().scratch.empty());
+}
+
+// No memory for a context's own table: an error, without a wait for a lock the
+// thread itself holds.
+static void context_without_memory() {
+  fake::capacity = 0;
+  int code = 0;
+  try {
+    ctx();
+  } catch (const PErr &e) {
+    code = e.code;
+  }
+  EXPECT(code == PASTA_E_NOMEM);
+}
+
+int main(int argc, char **argv) {
+  const std::string which = argc > 1 ? argv[1] : "";
+  if (which == "flush_while_contexts_are_looked_up") flush_while_contexts_are_looked_up();
+  else if (which == "context_without_memory") context_without_memory();
+  else return 2;
+  std::_Exit(0);
+}
