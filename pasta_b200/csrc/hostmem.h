@@ -191,9 +191,9 @@ Ctx &ctx() {
     g_dev = d;
   }
   std::lock_guard<std::mutex> lk(g_ctx_mu);
-  auto &c = g_ctx[g_dev];
-  if (!c) {
-    c.reset(new Ctx());
+  std::unique_ptr<Ctx> &slot = g_ctx[g_dev];
+  if (!slot) {
+    std::unique_ptr<Ctx> c(new Ctx());  // kept once it is whole
     c->dev = g_dev;
     CK(cudaSetDevice(g_dev));
     CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
@@ -207,9 +207,10 @@ Ctx &ctx() {
     }
     c->tw.alloc(t.size(), false);
     CK(cudaMemcpy(c->tw.p, t.data(), t.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    slot = std::move(c);
   }
-  CK(cudaSetDevice(c->dev));
-  return *c;
+  CK(cudaSetDevice(slot->dev));
+  return *slot;
 }
 
 // ------------------------------------------------------------ scratch pool

@@ -158,10 +158,32 @@ static void context_without_memory() {
   EXPECT(code == PASTA_E_NOMEM);
 }
 
+// A context that could not be made is made by the next call, whole.
+static void context_made_again() {
+  for (int what = 0; what < 3; what++) {
+    fake::streams_fail = what == 0;
+    fake::events_fail = what == 1;
+    if (what == 2) fake::capacity = 0;
+    int code = 0;
+    try {
+      ctx();
+    } catch (const PErr &e) {
+      code = e.code;
+    }
+    EXPECT(code != 0);
+    fake::streams_fail = fake::events_fail = false;
+    fake::capacity = 1ull << 40;
+  }
+  Ctx &C = ctx();
+  EXPECT(C.stream && C.side && C.fork && C.join && C.tw.p);
+  EXPECT(C.tw.p[0].x == 1.0f && C.tw.p[FFTN / 2].x == -1.0f);
+}
+
 int main(int argc, char **argv) {
   const std::string which = argc > 1 ? argv[1] : "";
   if (which == "flush_while_contexts_are_looked_up") flush_while_contexts_are_looked_up();
   else if (which == "context_without_memory") context_without_memory();
+  else if (which == "context_made_again") context_made_again();
   else return 2;
   std::_Exit(0);
 }

@@ -31,3 +31,7 @@ def _run(binary, case):
 @pytest.mark.parametrize("case", ["flush_while_contexts_are_looked_up", "context_without_memory"])
 def test_pool_is_given_back_when_memory_runs_out(binary, case):
     _run(binary, case)
+
+
+def test_context_that_failed_is_made_again(binary):
+    _run(binary, "context_made_again")
