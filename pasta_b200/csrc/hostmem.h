@@ -167,6 +167,24 @@ struct Stage {
   cudaEvent_t ev[2] = {};
   int at = 0;       // half in use
   size_t fill = 0;  // bytes used of it
+  // the buffer with both events, or nothing
+  bool ready() {
+    if (buf.p) return true;
+    HostBuf<unsigned char> b;
+    cudaEvent_t e[2] = {};
+    bool made = cudaMallocHost(&b.p, 2 * STAGE_HALF) == cudaSuccess;
+    if (!made) b.p = nullptr;
+    for (int k = 0; k < 2 && made; k++) made = cudaEventCreateWithFlags(&e[k], cudaEventDisableTiming) == cudaSuccess;
+    if (!made) {
+      cudaGetLastError();
+      for (cudaEvent_t x : e)
+        if (x) cudaEventDestroy(x);
+      return false;
+    }
+    std::swap(buf.p, b.p);
+    std::copy(e, e + 2, ev);
+    return true;
+  }
 };
 struct Ctx {
   int dev = 0;
@@ -308,18 +326,13 @@ void copy_threads(void *dst, const void *src, size_t n) {
 }
 
 // Copies between host arrays and the device through the staging buffer, in
-// order on the device's stream; pageable copies while another thread holds it.
+// order on the device's stream; pageable copies while another thread holds it
+// or when no page-locked memory is to be had.
 struct HostCopy {
   Ctx &C;
   std::unique_lock<std::mutex> lk;
   bool ok;
-  explicit HostCopy(Ctx &c) : C(c), lk(c.stage.mu, std::try_to_lock), ok(lk.owns_lock()) {
-    Stage &S = C.stage;
-    if (ok && !S.buf.p) {
-      S.buf.alloc(2 * STAGE_HALF);
-      for (auto &e : S.ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    }
-  }
+  explicit HostCopy(Ctx &c) : C(c), lk(c.stage.mu, std::try_to_lock), ok(lk.owns_lock() && c.stage.ready()) {}
   // room for n bytes (at most STAGE_HALF) in the current half, or the next one
   unsigned char *room(size_t n) {
     Stage &S = C.stage;

@@ -53,6 +53,7 @@ cudaError_t cudaMallocHost(void **p, size_t n) {
   *p = std::malloc(n);
   return cudaSuccess;
 }
+cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return cudaMallocHost(p, n); }
 cudaError_t cudaFreeHost(void *p) {
   std::free(p);
   return cudaSuccess;
@@ -179,11 +180,40 @@ static void context_made_again() {
   EXPECT(C.tw.p[0].x == 1.0f && C.tw.p[FFTN / 2].x == -1.0f);
 }
 
+// n bytes there and back through HostCopy, in one piece and in small pieces
+static void copies_agree(size_t n) {
+  std::vector<unsigned char> in(n), out(n, 0);
+  for (size_t i = 0; i < n; i++) in[i] = (unsigned char)(i * 131 + (i >> 9));
+  SBuf<unsigned char> d;
+  d.alloc(n);
+  HostCopy hc(ctx());
+  hc.up(d.p, in.data(), n / 3);
+  hc.up(d.p + n / 3, in.data() + n / 3, n - n / 3);
+  hc.down(out.data(), d.p, n);
+  EXPECT(in == out);
+}
+
+// Without page-locked memory, or without an event for it, copies go on
+// unstaged; staged again once both can be had.
+static void copies_without_staging() {
+  for (int what = 0; what < 2; what++) {
+    fake::pinned_fails = what == 0;
+    ctx();
+    fake::events_fail = what == 1;
+    for (size_t n : {(size_t)1000, (size_t)200000, (size_t)9 << 20}) copies_agree(n);
+    EXPECT(!ctx().stage.buf.p && !ctx().stage.ev[0] && !ctx().stage.ev[1]);
+    fake::pinned_fails = fake::events_fail = false;
+  }
+  for (size_t n : {(size_t)1000, (size_t)200000, (size_t)9 << 20}) copies_agree(n);
+  EXPECT(ctx().stage.buf.p && ctx().stage.ev[0] && ctx().stage.ev[1]);
+}
+
 int main(int argc, char **argv) {
   const std::string which = argc > 1 ? argv[1] : "";
   if (which == "flush_while_contexts_are_looked_up") flush_while_contexts_are_looked_up();
   else if (which == "context_without_memory") context_without_memory();
   else if (which == "context_made_again") context_made_again();
+  else if (which == "copies_without_staging") copies_without_staging();
   else return 2;
   std::_Exit(0);
 }

@@ -35,3 +35,7 @@ def test_pool_is_given_back_when_memory_runs_out(binary, case):
 
 def test_context_that_failed_is_made_again(binary):
     _run(binary, "context_made_again")
+
+
+def test_copies_go_on_without_page_locked_memory(binary):
+    _run(binary, "copies_without_staging")
