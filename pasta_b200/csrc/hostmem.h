@@ -15,7 +15,6 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -306,23 +305,25 @@ void scratch_put(void *p, size_t bytes, int dev) {
 // memcpy of large arrays by a few threads (one core moves 8-10 GB/s, less
 // into pages touched for the first time)
 void copy_threads(void *dst, const void *src, size_t n) {
-  const size_t parts = std::min<size_t>(4, n >> 20);
+  constexpr size_t MOST = 4;
+  const size_t parts = std::min(MOST, n >> 20);
   if (parts < 2) {
     std::memcpy(dst, src, n);
     return;
   }
-  std::vector<std::thread> th;
+  std::thread th[MOST];  // no allocation while threads run: nothing but a thread's start can fail
   const size_t per = (n / parts + 4095) & ~(size_t)4095;
   for (size_t k = 1; k < parts; k++) {
     const size_t o = k * per, m = k + 1 == parts ? n - o : per;
     try {
-      th.emplace_back([=] { std::memcpy((char *)dst + o, (const char *)src + o, m); });
-    } catch (const std::system_error &) {  // no thread to be had
+      th[k] = std::thread([=] { std::memcpy((char *)dst + o, (const char *)src + o, m); });
+    } catch (const std::exception &) {  // no thread, or no memory for one
       std::memcpy((char *)dst + o, (const char *)src + o, m);
     }
   }
   std::memcpy(dst, src, per);
-  for (auto &t : th) t.join();
+  for (auto &t : th)
+    if (t.joinable()) t.join();
 }
 
 // Copies between host arrays and the device through the staging buffer, in

@@ -105,6 +105,16 @@ cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
 cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
 }
 
+// the n-th host allocation of this thread from now on fails (0: none)
+static thread_local int new_countdown = 0;
+void *operator new(size_t n) {
+  if (new_countdown > 0 && --new_countdown == 0) throw std::bad_alloc();
+  if (void *p = std::malloc(n)) return p;
+  throw std::bad_alloc();
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, size_t) noexcept { std::free(p); }
+
 #define EXPECT(cond)                                                     \
   do {                                                                   \
     if (!(cond)) {                                                       \
@@ -208,12 +218,27 @@ static void copies_without_staging() {
   EXPECT(ctx().stage.buf.p && ctx().stage.ev[0] && ctx().stage.ev[1]);
 }
 
+// A copy by several threads is whole whichever of its host allocations fails.
+static void threads_without_host_memory() {
+  const size_t n = (4u << 20) + 4097;
+  std::vector<unsigned char> in(n), out(n);
+  for (size_t i = 0; i < n; i++) in[i] = (unsigned char)(i * 131 + (i >> 9));
+  for (int k = 0; k < 10; k++) {
+    std::fill(out.begin(), out.end(), 0);
+    new_countdown = k;
+    copy_threads(out.data(), in.data(), n);
+    new_countdown = 0;
+    EXPECT(in == out);
+  }
+}
+
 int main(int argc, char **argv) {
   const std::string which = argc > 1 ? argv[1] : "";
   if (which == "flush_while_contexts_are_looked_up") flush_while_contexts_are_looked_up();
   else if (which == "context_without_memory") context_without_memory();
   else if (which == "context_made_again") context_made_again();
   else if (which == "copies_without_staging") copies_without_staging();
+  else if (which == "threads_without_host_memory") threads_without_host_memory();
   else return 2;
   std::_Exit(0);
 }

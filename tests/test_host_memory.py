@@ -39,3 +39,7 @@ def test_context_that_failed_is_made_again(binary):
 
 def test_copies_go_on_without_page_locked_memory(binary):
     _run(binary, "copies_without_staging")
+
+
+def test_copy_threads_without_host_memory(binary):
+    _run(binary, "threads_without_host_memory")
