@@ -252,7 +252,7 @@ void scratch_flush(int dev) {
 }
 void *scratch_take(size_t bytes, size_t *got) {
   Ctx &C = ctx();
-  const size_t want = scratch_round(bytes);
+  const size_t want = bytes <= SCRATCH_BLOCK ? scratch_round(bytes) : bytes;  // no slack for blocks that are not kept
   *got = want;
   if (want <= SCRATCH_BLOCK) {
     std::lock_guard<std::mutex> lk(C.scratch_mu);
@@ -274,11 +274,12 @@ void *scratch_take(size_t bytes, size_t *got) {
   if (e != cudaSuccess) {
     cudaGetLastError();
     scratch_flush(-1);
-    e = cudaMalloc(&p, want);
+    *got = bytes;  // no slack either when memory is short
+    e = cudaMalloc(&p, bytes);
   }
   if (e != cudaSuccess) {
     cudaGetLastError();
-    fail(PASTA_E_NOMEM, "cudaMalloc of %zu bytes failed: %s", want, cudaGetErrorString(e));
+    fail(PASTA_E_NOMEM, "cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
   }
   return p;
 }

@@ -232,6 +232,24 @@ static void threads_without_host_memory() {
   }
 }
 
+// A buffer that fits the device's free memory exactly is had, small or large.
+static void exact_fits() {
+  ctx();
+  for (size_t n : {(size_t)1000, (size_t)9 << 20, ((size_t)60 << 20) + 1, (size_t)64 << 20, ((size_t)64 << 20) + 1,
+                   (size_t)1000 << 20, ((size_t)9 << 30) + 12}) {
+    fake::capacity = fake::used + n;
+    int code = 0;
+    try {
+      SBuf<char> b;
+      b.alloc(n);
+    } catch (const PErr &e) {
+      code = e.code;
+    }
+    EXPECT(code == 0);
+    scratch_flush(-1);
+  }
+}
+
 int main(int argc, char **argv) {
   const std::string which = argc > 1 ? argv[1] : "";
   if (which == "flush_while_contexts_are_looked_up") flush_while_contexts_are_looked_up();
@@ -239,6 +257,7 @@ int main(int argc, char **argv) {
   else if (which == "context_made_again") context_made_again();
   else if (which == "copies_without_staging") copies_without_staging();
   else if (which == "threads_without_host_memory") threads_without_host_memory();
+  else if (which == "exact_fits") exact_fits();
   else return 2;
   std::_Exit(0);
 }

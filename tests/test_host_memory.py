@@ -43,3 +43,7 @@ def test_copies_go_on_without_page_locked_memory(binary):
 
 def test_copy_threads_without_host_memory(binary):
     _run(binary, "threads_without_host_memory")
+
+
+def test_scratch_that_fits_exactly(binary):
+    _run(binary, "exact_fits")
