@@ -793,9 +793,10 @@ void run_evals(pasta_grid *g, const EvalArgs &a, cudaStream_t s) {
   o.full_window = a.full_window;
   o.rot = a.max_m > 1;
   o.may_unfuse = may_unfuse;
-  o.side = C.side;
-  o.fork = C.fork;
-  o.join = C.join;
+  const Lane &lane = s == C.cap.stream ? C.cap : C;
+  o.side = lane.side;
+  o.fork = lane.fork;
+  o.join = lane.join;
   for (int64_t off = 0; off < a.E; off += cap) {
     const int64_t cnt = std::min(cap, a.E - off);
     EvalBatch b = make_batch(g, a, off, cnt);
@@ -1105,9 +1106,9 @@ void batch_init(Batch &B, pasta_grid *g, const std::vector<StarInput> &in) {
   for (auto &e : B.ev) CK(cudaEventCreate(&e));
   if (!getenv("PASTA_NO_GRAPH")) {
     const int64_t k0 = kernel_launches();
-    CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    B.step_eager(s);
-    CK(cudaStreamEndCapture(s, &B.graph));
+    Capture cap(C);
+    B.step_eager(cap.stream());
+    cap.finish(&B.graph);
     CK(cudaGraphInstantiate(&B.exec, B.graph, 0));
     B.kernels_per_step = (int)(kernel_launches() - k0);
   }
@@ -2689,7 +2690,7 @@ int pasta_binary_fit(const pasta_grid *g_, const pasta_grid *cg, const pasta_dis
     hx.alloc((size_t)P * D);
     hcost.alloc(P);
     hest.alloc(P);
-    auto enqueue = [&]() {
+    auto enqueue = [&](cudaStream_t s) {
       CK(cudaMemcpyAsync(bs.labels.p, hx.p, (size_t)P * D * sizeof(double), cudaMemcpyHostToDevice, s));
       run_binary(g, cg, ds.p, hstar, bs, P, vs_max, true, nullptr, 0, s);
       CK(cudaMemcpyAsync(hcost.p, bs.cost.p, P * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -2701,21 +2702,13 @@ int pasta_binary_fit(const pasta_grid *g_, const pasta_grid *cg, const pasta_dis
       std::copy(x.begin(), x.end(), hx.p);
       if (try_graph) {
         try_graph = false;
-        CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        try {
-          enqueue();
-        } catch (...) {
-          cudaGraph_t dead = nullptr;
-          cudaStreamEndCapture(s, &dead);  // leave capture mode before the error propagates
-          if (dead) cudaGraphDestroy(dead);
-          cudaGetLastError();
-          throw;
-        }
-        CK(cudaStreamEndCapture(s, &gh.graph));
+        Capture cap(C);
+        enqueue(cap.stream());
+        cap.finish(&gh.graph);
         CK(cudaGraphInstantiate(&gh.exec, gh.graph, 0));
       }
       if (gh.exec) CK(cudaGraphLaunch(gh.exec, s));
-      else enqueue();
+      else enqueue(s);
       CK(cudaStreamSynchronize(s));
       std::copy(hcost.p, hcost.p + P, cost.begin());
       std::copy(hest.p, hest.p + P, est.begin());
@@ -3371,10 +3364,10 @@ int pasta_server_step(pasta_server *sv) {
       sv->graph_chunks = a.max_chunks;
       sv->graph_lin = a.lin_kp_mask;
       const int64_t k0 = kernel_launches();
-      CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-      launch_pso_update(g->d, sw, s);
-      run_evals(g, a, s);
-      launch_pso_best(sw, sv->W.ecost.p, sv->W.estatus.p, s);
+      Capture cap(C);
+      launch_pso_update(g->d, sw, cap.stream());
+      run_evals(g, a, cap.stream());
+      launch_pso_best(sw, sv->W.ecost.p, sv->W.estatus.p, cap.stream());
       // final refit (fitting.rs:436-440) of the swarms that finished in this
       // step: chi2 at the best label with the continuum parameters written
       EvalArgs r = a;
@@ -3386,8 +3379,8 @@ int pasta_server_step(pasta_server *sv) {
       r.status = sv->rf_status.p;
       r.params = sv->rf_params.p;
       r.param_stride = SERVER_REFIT_STRIDE;
-      run_evals(g, r, s);
-      CK(cudaStreamEndCapture(s, &sv->graph));
+      run_evals(g, r, cap.stream());
+      cap.finish(&sv->graph);
       sv->graph_kernels = kernel_launches() - k0;
       count_launch(-(int)sv->graph_kernels);  // counted again at every replay
       CK(cudaGraphInstantiate(&sv->exec, sv->graph, 0));

@@ -185,11 +185,25 @@ struct Stage {
     return true;
   }
 };
-struct Ctx {
-  int dev = 0;
-  cudaStream_t stream = nullptr;
-  cudaStream_t side = nullptr;                  // see PipelineOpts::side
+// A stream with its side stream (see PipelineOpts::side)
+struct Lane {
+  cudaStream_t stream = nullptr, side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
+  void make() {
+    CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    CK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+  }
+};
+// A device's context.  Calls are serialised per grid, so two grids' calls
+// enqueue on the lane at the same time; graphs are captured on a lane of their
+// own (Capture), or what another thread enqueues, copies or waits for
+// meanwhile would become part of the graph or end the capture.
+struct Ctx : Lane {
+  int dev = 0;
+  Lane cap;
+  std::mutex cap_mu;
   DBuf<float2> tw;  // W_2048^k
   Stage stage;
   std::mutex scratch_mu;
@@ -213,10 +227,8 @@ Ctx &ctx() {
     std::unique_ptr<Ctx> c(new Ctx());  // kept once it is whole
     c->dev = g_dev;
     CK(cudaSetDevice(g_dev));
-    CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-    CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
-    CK(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming));
+    c->make();
+    c->cap.make();
     std::vector<float2> t(FFTN);
     for (int k = 0; k < FFTN; k++) {
       double a = -2.0 * M_PI * (double)k / (double)FFTN;
@@ -229,6 +241,34 @@ Ctx &ctx() {
   CK(cudaSetDevice(slot->dev));
   return *slot;
 }
+
+// One graph capture on the device's capture lane (one at a time); ends the
+// capture when the scope is left without finish().
+class Capture {
+  Ctx &C;
+  std::lock_guard<std::mutex> lk;
+  bool open = false;
+
+ public:
+  explicit Capture(Ctx &c) : C(c), lk(c.cap_mu) {
+    CK(cudaStreamBeginCapture(C.cap.stream, cudaStreamCaptureModeThreadLocal));
+    open = true;
+  }
+  Capture(const Capture &) = delete;
+  Capture &operator=(const Capture &) = delete;
+  ~Capture() {
+    if (!open) return;
+    cudaGraph_t dead = nullptr;
+    cudaStreamEndCapture(C.cap.stream, &dead);
+    if (dead) cudaGraphDestroy(dead);
+    cudaGetLastError();
+  }
+  cudaStream_t stream() const { return C.cap.stream; }
+  void finish(cudaGraph_t *graph) {
+    open = false;
+    CK(cudaStreamEndCapture(C.cap.stream, graph));
+  }
+};
 
 // ------------------------------------------------------------ scratch pool
 int scratch_device() { return ctx().dev; }

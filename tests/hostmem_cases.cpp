@@ -19,14 +19,31 @@ std::vector<size_t> asked;               // sizes of all device allocations, in 
 std::atomic<bool> pinned_fails{false}, events_fail{false}, streams_fail{false};
 std::atomic<uintptr_t> next_handle{16};
 std::set<cudaEvent_t> events;
+std::set<cudaStream_t> capturing;
+std::atomic<int> into_capture{0};        // calls that landed in a capture, or that end one
 cudaError_t last = cudaSuccess;
 cudaError_t set(cudaError_t e) {
   if (e != cudaSuccess) last = e;
   return e;
 }
+bool in_capture(cudaStream_t s) {
+  std::lock_guard<std::mutex> lk(mu);
+  const bool c = capturing.count(s);
+  into_capture += c;
+  return c;
+}
 }  // namespace fake
 
 extern "C" {
+cudaError_t cudaStreamBeginCapture(cudaStream_t s, cudaStreamCaptureMode) {
+  std::lock_guard<std::mutex> lk(fake::mu);
+  return fake::capturing.insert(s).second ? cudaSuccess : fake::set(cudaErrorIllegalState);
+}
+cudaError_t cudaStreamEndCapture(cudaStream_t s, cudaGraph_t *g) {
+  std::lock_guard<std::mutex> lk(fake::mu);
+  *g = (cudaGraph_t)(fake::next_handle += 16);
+  return fake::capturing.erase(s) ? cudaSuccess : fake::set(cudaErrorIllegalState);
+}
 cudaError_t cudaMalloc(void **p, size_t n) {
   std::lock_guard<std::mutex> lk(fake::mu);
   fake::asked.push_back(n);
@@ -69,11 +86,13 @@ cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) {
   return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t st) {
-  if (!st) return fake::set(cudaErrorInvalidResourceHandle);
+  if (!st || fake::in_capture(st)) return fake::set(cudaErrorInvalidResourceHandle);
   std::memcpy(d, s, n);
   return cudaSuccess;
 }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+  return fake::in_capture(s) ? fake::set(cudaErrorStreamCaptureUnsupported) : cudaSuccess;
+}
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
   if (fake::streams_fail) return fake::set(cudaErrorMemoryAllocation);
   *s = (cudaStream_t)(fake::next_handle += 16);
@@ -91,7 +110,8 @@ cudaError_t cudaEventDestroy(cudaEvent_t e) {
   std::lock_guard<std::mutex> lk(fake::mu);
   return fake::events.erase(e) ? cudaSuccess : fake::set(cudaErrorInvalidResourceHandle);
 }
-cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) {
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+  fake::in_capture(s);
   std::lock_guard<std::mutex> lk(fake::mu);
   return fake::events.count(e) ? cudaSuccess : fake::set(cudaErrorInvalidResourceHandle);
 }
@@ -250,6 +270,45 @@ static void exact_fits() {
   }
 }
 
+// Another thread's copies and pool waits while a graph is captured stay out of
+// the capture; captures come one at a time; one left by an exception is ended.
+static void captures_are_alone() {
+  Ctx &C = ctx();
+  for (size_t n : {(size_t)1000, (size_t)5 << 20}) copies_agree(n);
+  std::thread rival;
+  std::atomic<bool> second{false};
+  {
+    Capture cap(C);
+    EXPECT(cap.stream() != C.stream && cap.stream() != C.side);
+    std::thread([] {
+      for (int k = 0; k < 3; k++)
+        for (size_t n : {(size_t)1000, (size_t)200000, (size_t)9 << 20}) copies_agree(n);
+    }).join();
+    rival = std::thread([&] {
+      Capture again(ctx());
+      second = true;
+      cudaGraph_t g = nullptr;
+      again.finish(&g);
+    });
+    std::this_thread::sleep_for(std::chrono::milliseconds(50));
+    EXPECT(!second);
+    cudaGraph_t g = nullptr;
+    cap.finish(&g);
+    EXPECT(g);
+  }
+  rival.join();
+  EXPECT(second);
+  try {
+    Capture cap(C);
+    fail(PASTA_E_INTERNAL, "a launch that failed");
+  } catch (const PErr &) {
+  }
+  EXPECT(fake::capturing.empty() && fake::into_capture == 0);
+  Capture cap(C);
+  cudaGraph_t g = nullptr;
+  cap.finish(&g);
+}
+
 int main(int argc, char **argv) {
   const std::string which = argc > 1 ? argv[1] : "";
   if (which == "flush_while_contexts_are_looked_up") flush_while_contexts_are_looked_up();
@@ -258,6 +317,7 @@ int main(int argc, char **argv) {
   else if (which == "copies_without_staging") copies_without_staging();
   else if (which == "threads_without_host_memory") threads_without_host_memory();
   else if (which == "exact_fits") exact_fits();
+  else if (which == "captures_are_alone") captures_are_alone();
   else return 2;
   std::_Exit(0);
 }

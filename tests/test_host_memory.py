@@ -47,3 +47,7 @@ def test_copy_threads_without_host_memory(binary):
 
 def test_scratch_that_fits_exactly(binary):
     _run(binary, "exact_fits")
+
+
+def test_graph_captures_are_alone(binary):
+    _run(binary, "captures_are_alone")
