@@ -3379,6 +3379,8 @@ int pasta_server_step(pasta_server *sv) {
       r.status = sv->rf_status.p;
       r.params = sv->rf_params.p;
       r.param_stride = SERVER_REFIT_STRIDE;
+      r.lin_group = 1;  // one evaluation per star, as in final_refit
+      r.star_len = 1;
       run_evals(g, r, cap.stream());
       cap.finish(&sv->graph);
       sv->graph_kernels = kernel_launches() - k0;

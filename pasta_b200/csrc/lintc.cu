@@ -199,6 +199,8 @@ __global__ void __launch_bounds__(LT_T) k_linear_tc(EvalBatch b) {
   const bool member = p < LG && e < b.E;
   const EvalPrep *P = member ? &b.prep[e] : nullptr;
   const bool live = member && P->status == 0 && P->star == star && !st.cont_bad;
+  // most groups of a server's refit have nothing to do in most steps
+  if (!__syncthreads_or(live)) return;
   const float *mod = live ? lt_model_row(b, *P, e) : nullptr;
   const float *flux = st.flux, *var = st.var, *q = st.q, *qt = st.qt;
   constexpr int HALF = KP / 2;
