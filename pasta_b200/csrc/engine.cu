@@ -1499,7 +1499,7 @@ void tune_direct(pasta_grid *g) {
       double *q = &lab[(size_t)i * 5];
       q[0] = t; q[1] = mh; q[2] = lg; q[3] = lo; q[4] = 0.0;
     }
-    CK(cudaMemcpy(dl.p, lab.data(), lab.size() * sizeof(double), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(dl.p, lab.data(), lab.size() * sizeof(double), cudaMemcpyHostToDevice, s));
     EvalArgs a;
     a.stars = ds.p;
     a.labels = dl.p;
@@ -1600,7 +1600,7 @@ void tune_interp_tc(pasta_grid *g) {
       x[3] = 0.0;
       x[4] = 0.0;
     }
-    CK(cudaMemcpy(dl.p, lab.data(), lab.size() * sizeof(double), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(dl.p, lab.data(), lab.size() * sizeof(double), cudaMemcpyHostToDevice, s));
     EvalArgs a;
     a.stars = ds.p;
     a.labels = dl.p;
@@ -3227,7 +3227,7 @@ void server_rebuild(pasta_server *sv, int Pmax) {
   for (int i = 0; i < sv->slots; i++) ident[i] = i;
   sv->rf_star.upload(ident);
   sv->rf_flag.alloc(sv->slots);
-  CK(cudaMemset(sv->rf_flag.p, 0, sv->slots * sizeof(int)));
+  CK(cudaMemsetAsync(sv->rf_flag.p, 0, sv->slots * sizeof(int), scratch_stream()));
   sv->rf_status.alloc(sv->slots);
   sv->rf_cost.alloc(sv->slots);
   sv->rf_params.alloc((size_t)sv->slots * SERVER_REFIT_STRIDE);

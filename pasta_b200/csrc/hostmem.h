@@ -61,6 +61,14 @@ int scratch_device();
 cudaStream_t scratch_stream();
 void scratch_flush(int dev);
 
+// Copies a host array to the device and waits for it.  cudaMemcpy returns when
+// a pageable source has been staged, and what it still has under way is on the
+// legacy stream, which the library's non-blocking streams do not wait for.
+inline void copy_to_device(void *dst, const void *src, size_t n) {
+  CK(cudaMemcpy(dst, src, n, cudaMemcpyHostToDevice));
+  CK(cudaStreamSynchronize(cudaStreamLegacy));
+}
+
 // POOL: scratch of one call or fit (see scratch_take); its uploads are ordered
 // on the device's stream
 template <class T, bool POOL = false>
@@ -111,7 +119,7 @@ struct DBuf {
     alloc(count);
     if (!count) return;
     if (POOL) CK(cudaMemcpyAsync(p, h, count * sizeof(T), cudaMemcpyHostToDevice, scratch_stream()));
-    else CK(cudaMemcpy(p, h, count * sizeof(T), cudaMemcpyHostToDevice));
+    else copy_to_device(p, h, count * sizeof(T));
   }
   void upload(const std::vector<T> &v) { upload(v.data(), v.size()); }
 };
@@ -235,7 +243,7 @@ Ctx &ctx() {
       t[k] = make_float2((float)std::cos(a), (float)std::sin(a));
     }
     c->tw.alloc(t.size(), false);
-    CK(cudaMemcpy(c->tw.p, t.data(), t.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    copy_to_device(c->tw.p, t.data(), t.size() * sizeof(float2));
     slot = std::move(c);
   }
   CK(cudaSetDevice(slot->dev));

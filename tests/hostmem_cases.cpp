@@ -20,6 +20,7 @@ std::atomic<bool> pinned_fails{false}, events_fail{false}, streams_fail{false};
 std::atomic<uintptr_t> next_handle{16};
 std::set<cudaEvent_t> events;
 std::set<cudaStream_t> capturing;
+std::atomic<int> legacy_pending{0};      // copies on the legacy stream nothing has waited for
 std::atomic<int> into_capture{0};        // calls that landed in a capture, or that end one
 cudaError_t last = cudaSuccess;
 cudaError_t set(cudaError_t e) {
@@ -83,6 +84,7 @@ cudaError_t cudaGetLastError(void) {
 const char *cudaGetErrorString(cudaError_t) { return "stand-in error"; }
 cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) {
   std::memcpy(d, s, n);
+  fake::legacy_pending++;
   return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t st) {
@@ -91,6 +93,7 @@ cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cu
   return cudaSuccess;
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+  if (!s || s == cudaStreamLegacy) fake::legacy_pending = 0;
   return fake::in_capture(s) ? fake::set(cudaErrorStreamCaptureUnsupported) : cudaSuccess;
 }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
@@ -309,6 +312,16 @@ static void captures_are_alone() {
   cap.finish(&g);
 }
 
+// Uploads are complete when they return: nothing orders the library's streams
+// behind the legacy stream.
+static void uploads_are_waited_for() {
+  ctx();
+  EXPECT(fake::legacy_pending == 0);
+  DBuf<int> a;
+  a.upload(std::vector<int>(1000, 3));
+  EXPECT(fake::legacy_pending == 0 && a.p[999] == 3);
+}
+
 int main(int argc, char **argv) {
   const std::string which = argc > 1 ? argv[1] : "";
   if (which == "flush_while_contexts_are_looked_up") flush_while_contexts_are_looked_up();
@@ -318,6 +331,7 @@ int main(int argc, char **argv) {
   else if (which == "threads_without_host_memory") threads_without_host_memory();
   else if (which == "exact_fits") exact_fits();
   else if (which == "captures_are_alone") captures_are_alone();
+  else if (which == "uploads_are_waited_for") uploads_are_waited_for();
   else return 2;
   std::_Exit(0);
 }

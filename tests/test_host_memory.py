@@ -51,3 +51,7 @@ def test_scratch_that_fits_exactly(binary):
 
 def test_graph_captures_are_alone(binary):
     _run(binary, "captures_are_alone")
+
+
+def test_uploads_are_waited_for(binary):
+    _run(binary, "uploads_are_waited_for")
