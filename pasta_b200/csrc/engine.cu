@@ -1034,10 +1034,10 @@ struct Batch {
   double t0 = 0;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+  int64_t graph_gen = -1;  // workspace the graph was captured with
   cudaEvent_t ev[12] = {};
   ~Batch() {
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
+    drop_graph();
     for (auto &e : ev)
       if (e) cudaEventDestroy(e);
   }
@@ -1045,6 +1045,27 @@ struct Batch {
     launch_pso_update(g->d, sw, s);
     run_evals(g, a, s);
     launch_pso_best(sw, W.ecost.p, W.estatus.p, s);
+  }
+  void drop_graph() {
+    if (exec) cudaGraphExecDestroy(exec);
+    if (graph) cudaGraphDestroy(graph);
+    exec = nullptr;
+    graph = nullptr;
+  }
+  // The workspace and the step's graph: made at the first call, and again when
+  // another call on the grid has moved the workspace between two steps.
+  void ready() {
+    ensure_workspace(g, a.E, a.max_nobs);
+    if (exec && graph_gen == g->ws.gen) return;
+    drop_graph();
+    if (getenv("PASTA_NO_GRAPH")) return;
+    const int64_t k0 = kernel_launches();
+    Capture cap(ctx());
+    step_eager(cap.stream());
+    cap.finish(&graph);
+    CK(cudaGraphInstantiate(&exec, graph, 0));
+    graph_gen = g->ws.gen;
+    kernels_per_step = (int)(kernel_launches() - k0);
   }
 };
 
@@ -1102,16 +1123,8 @@ void batch_init(Batch &B, pasta_grid *g, const std::vector<StarInput> &in) {
   star_kinds(B.ss.h, a);
   a.lin_group = B.Pmax <= 128 ? B.Pmax : 0;  // star s owns evaluations [s Pmax, (s + 1) Pmax)
   a.star_len = B.Pmax;
-  ensure_workspace(g, (int64_t)E, a.max_nobs);
   for (auto &e : B.ev) CK(cudaEventCreate(&e));
-  if (!getenv("PASTA_NO_GRAPH")) {
-    const int64_t k0 = kernel_launches();
-    Capture cap(C);
-    B.step_eager(cap.stream());
-    cap.finish(&B.graph);
-    CK(cudaGraphInstantiate(&B.exec, B.graph, 0));
-    B.kernels_per_step = (int)(kernel_launches() - k0);
-  }
+  B.ready();
 }
 
 // Launch n PSO steps; returns the device time between CUDA events recorded
@@ -1121,6 +1134,7 @@ double batch_steps(Batch &B, int n, double *trace) {
   cudaStream_t s = C.stream;
   std::vector<double> tx, tc;
   const int Ptr = B.pp.empty() ? 0 : B.pp[0].P;
+  B.ready();
   CK(cudaEventRecord(B.ev[0], s));
   for (int k = 0; k < n; k++) {
     if (B.exec) CK(cudaGraphLaunch(B.exec, s));
@@ -1157,6 +1171,7 @@ void batch_profile_step(Batch &B, double *out) {
   cudaStream_t s = C.stream;
   pasta_grid *g = B.g;
   const EvalArgs &a = B.a;
+  B.ready();
   if (a.E > g->ws.cap) fail(PASTA_E_UNSUPPORTED, "profiled step needs the batch in one workspace");
   EvalBatch b = make_batch(g, a, 0, a.E);
   int may_unfuse;
