@@ -21,7 +21,7 @@ COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=o
           "-I" + os.path.join(ROOT, "include")]
 UNITS = [("prep.cu", ["-fmad=false"]), ("kernels.cu", []), ("broaden.cu", []), ("chunk.cu", []), ("binary.cu", ["-fmad=false"]), ("lintc.cu", []), ("interp_tc.cu", []),
          ("engine.cu", []), ("noalloc.cu", [])]
-DEPS = ["common.cuh", "device.cuh", "fft.cuh", "hostmem.h", "kernels.h"]
+DEPS = ["common.cuh", "device.cuh", "fft.cuh", "hostmem.h", "kernels.h", "noalloc_layout.h"]
 
 
 def _nvcc():

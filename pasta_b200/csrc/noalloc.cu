@@ -32,6 +32,7 @@
 #include "../../include/pasta_b200.h"
 #include "common.cuh"
 #include "kernels.h"
+#include "noalloc_layout.h"
 
 namespace pb {
 int internal_eval_view(const pasta_grid *g, const pasta_dispersion *d, const pasta_continuum *c, const float *flux,
@@ -44,7 +45,6 @@ using namespace pb;
 
 namespace {
 
-constexpr size_t NOALLOC_SCRATCH_BYTES = 32u << 20;
 constexpr int MAX_DEVICES = 64;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
@@ -66,19 +66,6 @@ struct ErrSink {
   }
   ErrSink &operator=(const char *m) { return *this = std::string(m); }
 } g_noalloc_err;
-
-size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
-
-// bytes of scratch one label needs: prep record, rotation half spectra
-// (alone and times the instrument spectrum),
-// eval->star index, the two spectrum rows, the broadening block bounds and
-// the partial chi2 sums
-size_t per_label_bytes(int64_t stride, int bnd_stride) {
-  return align256(sizeof(EvalPrep)) + 2 * align256(1025 * sizeof(float2)) + align256(sizeof(int)) +
-         2 * align256((size_t)stride * sizeof(float)) + align256((size_t)bnd_stride * sizeof(int)) +
-         align256((size_t)MAX_CHUNKS * sizeof(double)) +
-         align256(sizeof(GroupRec)) + align256(sizeof(int));
-}
 
 int setup_device(int dev, DeviceSetup **out) {
   std::lock_guard<std::mutex> lk(g_setup_mu);
@@ -170,10 +157,7 @@ extern "C" int pasta_chi2_noalloc(const pasta_grid *g, const pasta_dispersion *d
   if (L == 0) return PASTA_OK;  // nothing to evaluate, like pasta_chi2
   stride = std::max<int64_t>(stride, (n + 63) / 64 * 64);  // rows also hold the model at the observed pixels
   const int bstr = bnd_stride_for(G.npx);
-  // the star record, and the group slots of a partly filled last segment
-  const size_t fixed = align256(sizeof(DevStar)) + align256((size_t)(SEG - 1) * sizeof(GroupRec)) + 256;
-  const size_t per = per_label_bytes(stride, bstr);
-  const int64_t max_labels = NOALLOC_SCRATCH_BYTES > fixed ? (int64_t)((NOALLOC_SCRATCH_BYTES - fixed) / per) : 0;
+  const int64_t max_labels = noalloc_max_labels(stride, bstr);
   if (L > max_labels) {
     char buf[256];
     snprintf(buf, sizeof buf,
@@ -198,31 +182,10 @@ extern "C" int pasta_chi2_noalloc(const pasta_grid *g, const pasta_dispersion *d
   DeviceSetup *S = nullptr;
   rc = setup_device(dev, &S);
   if (rc) return rc;
-  // carve the scratch
-  unsigned char *p = S->scratch;
-  DevStar *dstar = (DevStar *)p;
-  p += fixed;
-  EvalPrep *prep = (EvalPrep *)p;
-  p += align256(sizeof(EvalPrep) * (size_t)L);
-  float2 *H = (float2 *)p;
-  p += align256(1025 * sizeof(float2) * (size_t)L);
-  float2 *HG = (float2 *)p;
-  p += align256(1025 * sizeof(float2) * (size_t)L);
-  int *eval_star = (int *)p;
-  p += align256(sizeof(int) * (size_t)L);
-  float *A = (float *)p;
-  p += align256((size_t)stride * sizeof(float) * (size_t)L);
-  float *B = (float *)p;
-  p += align256((size_t)stride * sizeof(float) * (size_t)L);
-  int *bnd = (int *)p;
-  p += align256((size_t)bstr * sizeof(int) * (size_t)L);
-  double *cpart = (double *)p;
-  p += align256((size_t)MAX_CHUNKS * sizeof(double) * (size_t)L);
-  // SEG group slots per segment of SEG labels: L rounded up to SEG
-  const int64_t Lseg = (L + SEG - 1) / SEG * SEG;
-  GroupRec *grec = (GroupRec *)p;
-  p += align256(sizeof(GroupRec) * (size_t)Lseg);
-  int *gcount = (int *)p;
+  const NoallocLayout at = noalloc_layout(L, stride, bstr);
+  auto part = [&](size_t offset) { return S->scratch + offset; };
+  DevStar *dstar = (DevStar *)part(at.star);
+  int *eval_star = (int *)part(at.eval_star);
   cudaStream_t s = (cudaStream_t)stream;
   k_noalloc_init<<<(unsigned)((L + 255) / 256), 256, 0, s>>>(star, dstar, eval_star, (int)L);
   EvalBatch b{};
@@ -230,11 +193,11 @@ extern "C" int pasta_chi2_noalloc(const pasta_grid *g, const pasta_dispersion *d
   b.labels = labels;
   b.eval_star = eval_star;
   b.stars = dstar;
-  b.prep = prep;
-  b.H = H;
-  b.HG = HG;
-  b.bufA = A;
-  b.bufB = B;
+  b.prep = (EvalPrep *)part(at.prep);
+  b.H = (float2 *)part(at.H);
+  b.HG = (float2 *)part(at.HG);
+  b.bufA = (float *)part(at.A);
+  b.bufB = (float *)part(at.B);
   b.stride = stride;
   b.cost = out;
   b.status = status;
@@ -250,11 +213,11 @@ extern "C" int pasta_chi2_noalloc(const pasta_grid *g, const pasta_dispersion *d
   b.other_cont = star.cont_kind == CONT_CHUNK ? 0 : 1;
   b.obs_epi = 1;
   b.late_resample = 1;
-  b.bnd = bnd;
+  b.bnd = (int *)part(at.bnd);
   b.bnd_stride = bstr;
-  b.cpart = cpart;
-  b.grec = grec;
-  b.gcount = gcount;
+  b.cpart = (double *)part(at.cpart);
+  b.grec = (GroupRec *)part(at.grec);
+  b.gcount = (int *)part(at.gcount);
   launch_pipeline(G, b, S->twiddle, o, s);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
