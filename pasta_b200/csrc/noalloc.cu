@@ -9,7 +9,7 @@
 // buffers the caller already owns.  The evaluation workspace lives in the
 // file-scope array g_noalloc_scratch below.
 //
-// The array is NOALLOC_SCRATCH_BYTES (32 MiB).  Every GPU that loads the
+// The array is NOALLOC_SCRATCH_BYTES (32 MiB and 4 KiB).  Every GPU that loads the
 // library holds it until the process exits.  All calls share it and it keeps
 // the last call's contents.  No part of it has to start at zero: every stage
 // writes the rows it later reads.  Calls whose work overlaps on the GPU race

@@ -10,7 +10,9 @@
 
 namespace pb {
 
-constexpr size_t NOALLOC_SCRATCH_BYTES = 32u << 20;
+// 32 MiB, and what the group records have grown by since the limits on the
+// label count were first set
+constexpr size_t NOALLOC_SCRATCH_BYTES = (32u << 20) + 4096;
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
