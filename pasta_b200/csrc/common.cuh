@@ -187,6 +187,9 @@ PB_HD int find_neighbors(const double *v, int n, double x, int left, int right, 
     else if (i == right) { out[0] = i - 2; out[1] = i - 1; out[2] = i; out[3] = -1; }
     else { out[0] = i - 2; out[1] = i - 1; out[2] = i; out[3] = i + 1; }
   }
+  // past the axis: then there are two neighbours at most, too few for any
+  // interpolation (an index panic in the reference)
+  if (out[2] >= n || out[3] >= n) return S_NEIGHBORS;
   return S_OK;
 }
 
