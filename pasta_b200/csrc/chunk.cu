@@ -40,8 +40,14 @@ __device__ __forceinline__ float poly_eval(const float *coef, float x) {
 //
 // Divisions are multiplications by the reciprocal (at most 2 ulp; the sums
 // run over thousands of such terms).  The fast reciprocal takes a divisor
-// below 2^-126 (a variance in faint absolute units) as zero: a sum that comes
-// out infinite or NaN is formed again with divisions, plainly.
+// below 2^-126 (a variance in faint absolute units) as zero, so the walks also
+// come with divisions (DIV): stars with such variances take them for the
+// residuals from the start (faint_star), and a piece whose sum comes out
+// infinite or NaN is formed again with them if one of its divisors is that
+// small (any other cause gives the same sum either way).  A chi2 call of 2,000
+// evaluations of 60,000 pixels, degree 5: 0.91 ms; of a star with variances
+// around 1e-40 1.01 ms and with a NaN pixel in every piece 1.11 ms (1.36 and
+// 2.06 ms with every piece whose sum is not finite formed again pixel by pixel).
 //
 // Order of the sums: a range of pixels is cut into blocks of 32 x CU pixels;
 // lane l of the warp that takes a block adds its pixels l + 32 u, u < CU, in
@@ -75,6 +81,28 @@ __device__ __forceinline__ float rcp_ftz(float x) {
 }
 // 1 / x of two pixels, with divisors below 2^-126 taken as zero
 __device__ __forceinline__ float2 rcp2(float2 x) { return make_float2(rcp_ftz(x.x), rcp_ftz(x.y)); }
+
+// a / b of two pixels, any b that is not 0
+__device__ __forceinline__ float2 div2(float2 a, float2 b) { return make_float2(__fdividef(a.x, b.x), __fdividef(a.y, b.y)); }
+
+// whether one of p[i0, i1) is not 0 and below 2^-126, by a warp
+__device__ __forceinline__ bool any_subnormal(const float *__restrict__ p, int i0, int i1, int lane) {
+  bool any = false;
+#pragma unroll 8
+  for (int i = i0 + lane; i < i1; i += 32) {
+    const float a = fabsf(__ldg(p + i));
+    any |= a > 0.0f && a < 1.17549435e-38f;
+  }
+  return __any_sync(0xffffffffu, any);
+}
+// whether this thread's sample of the star's variances (256 over the spectrum,
+// whatever the number of threads) is near or below 2^-126
+__device__ __forceinline__ bool faint_star(const DevStar &st) {
+  const int t = threadIdx.x;
+  if (t >= 256) return false;
+  const float v = fabsf(__ldg(st.var + (long long)t * st.n_obs / 256));
+  return v > 0.0f && v < 1e-35f;
+}
 
 // Two blocks' loads for one lane: (first block, second block) at the lane's
 // u-th pixel.  INNER: every pixel of both blocks exists.  Otherwise pixels
@@ -111,7 +139,7 @@ __device__ __forceinline__ int blocks_of(int a0, int a1, int per) { return a1 > 
 
 // Adds the lane's share of sum_i P_k(x_i) flux_i / model_i over the blocks
 // [j0, j1) of [a0, a1) to z, for NE models of one star.
-template <int K, int NE>
+template <int K, int NE, bool DIV>
 __device__ __forceinline__ void moments_walk(const float *__restrict__ flux, const float *const (&mod)[NE],
                                              const float *__restrict__ xs, int a0, int a1, int j0, int j1, int lane,
                                              double (&z)[NE][K]) {
@@ -134,16 +162,22 @@ __device__ __forceinline__ void moments_walk(const float *__restrict__ flux, con
       }
 #pragma unroll
       for (int u = 0; u < 4; u++) {
-        const float2 f = ld.mask(fl[u], u0 + u), x = xf[u];
-        float2 y[NE];
+        const float2 f = ld.mask(fl[u], u0 + u);
+        [[maybe_unused]] const float2 x = xf[u];
+        [[maybe_unused]] float2 y[NE];
 #pragma unroll
         for (int n = 0; n < NE; n++) {
-          const float2 r = ld.mask(rcp2(md[n][u]), u0 + u);
-          if constexpr (K == 1) {
-            zp[n][0] = __ffma2_rn(f, r, zp[n][0]);
-          } else {
-            y[n] = __fmul2_rn(f, r);
+          if constexpr (DIV) {
+            y[n] = ld.mask(div2(f, md[n][u]), u0 + u);
             zp[n][0] = __fadd2_rn(zp[n][0], y[n]);
+          } else {
+            const float2 r = ld.mask(rcp2(md[n][u]), u0 + u);
+            if constexpr (K == 1) {
+              zp[n][0] = __ffma2_rn(f, r, zp[n][0]);
+            } else {
+              y[n] = __fmul2_rn(f, r);
+              zp[n][0] = __fadd2_rn(zp[n][0], y[n]);
+            }
           }
         }
         if constexpr (K > 1) {
@@ -196,46 +230,65 @@ __device__ __forceinline__ double warp_sum_vec(const double (&z)[K], int lane) {
   return v[0];
 }
 
+// Piece p of chunk c.  The chunk's pixels below the previous chunk's stop take
+// the upper-chunk coordinate xb; the pieces cut the blocks of both ranges,
+// taken one after the other, at even block numbers (pairs of blocks).
+template <int K>
+struct MomentPiece {
+  int lo, split, hi, bb, ba, nb, g0, g1;
+  __device__ __forceinline__ MomentPiece(const DevStar &st, int c, int p) {
+    constexpr int PER = 32 * chunk_cu<K>();
+    lo = st.cstart[c];
+    hi = st.cstop[c];
+    const int prev = c > 0 ? st.cstop[c - 1] : -1;
+    split = c > 0 ? min(max(prev, lo), hi) : lo;
+    bb = blocks_of(lo, split, PER);
+    ba = blocks_of(split, hi, PER);
+    nb = (bb + 1) / 2;
+    const int n = nb + (ba + 1) / 2;
+    g0 = n * p / CHUNK_PIECES;
+    g1 = n * (p + 1) / CHUNK_PIECES;
+  }
+  template <int NE, bool DIV>
+  __device__ __forceinline__ void sums(const DevStar &st, const float *const (&mod)[NE], int lane, double (&t)[NE]) const {
+    double z[NE][K];
+#pragma unroll
+    for (int q = 0; q < NE; q++)
+#pragma unroll
+      for (int k = 0; k < K; k++) z[q][k] = 0.0;
+    moments_walk<K, NE, DIV>(st.flux, mod, st.xb, lo, split, 2 * min(g0, nb), min(2 * min(g1, nb), bb), lane, z);
+    moments_walk<K, NE, DIV>(st.flux, mod, st.xa, split, hi, 2 * max(g0 - nb, 0), min(2 * max(g1 - nb, 0), ba), lane, z);
+#pragma unroll
+    for (int q = 0; q < NE; q++) t[q] = warp_sum_vec<K>(z[q], lane);
+  }
+};
+
+// The lane's slot of the moments of a piece whose sums t came out infinite or
+// NaN: formed with divisions if a model pixel is that small.  Not inlined, so
+// that it takes no registers from the common path.
+template <int K>
+__device__ __noinline__ double chunk_moments_again(const DevStar &st, const float *model, int c, int p, double t) {
+  constexpr int PER = 32 * chunk_cu<K>();
+  const int lane = threadIdx.x & 31;
+  const MomentPiece<K> P(st, c, p);
+  const int i0 = P.g0 < P.nb ? P.lo + 2 * PER * P.g0 : P.split + 2 * PER * (P.g0 - P.nb);
+  const int i1 = P.g1 < P.nb ? P.lo + 2 * PER * P.g1 : P.g1 == P.nb ? P.split : min(P.hi, P.split + 2 * PER * (P.g1 - P.nb));
+  if (!any_subnormal(model, i0, i1, lane)) return t;
+  const float *const mod[1] = {model};
+  double s[1];
+  P.template sums<1, true>(st, mod, lane, s);
+  return s[0];
+}
+
 // Moments of piece p of chunk c by one warp, for NE models: the lane's slot
-// of them (chunk_slot).  The chunk's pixels below the previous chunk's stop
-// take the upper-chunk coordinate xb.
+// of them (chunk_slot).
 template <int K, int NE>
 __device__ __forceinline__ void chunk_moments(const DevStar &st, const float *const (&mod)[NE], int c, int p, int lane,
                                               double (&t)[NE]) {
-  constexpr int PER = 32 * chunk_cu<K>();
-  const int lo = st.cstart[c], hi = st.cstop[c], prev = c > 0 ? st.cstop[c - 1] : -1;
-  const int split = c > 0 ? min(max(prev, lo), hi) : lo;
-  // the pieces cut the blocks of both ranges, taken one after the other, at
-  // even block numbers (pairs of blocks)
-  const int bb = blocks_of(lo, split, PER), ba = blocks_of(split, hi, PER), nb = (bb + 1) / 2, n = nb + (ba + 1) / 2;
-  const int g0 = n * p / CHUNK_PIECES, g1 = n * (p + 1) / CHUNK_PIECES;
-  double z[NE][K];
+  MomentPiece<K>(st, c, p).template sums<NE, false>(st, mod, lane, t);
 #pragma unroll
   for (int q = 0; q < NE; q++)
-#pragma unroll
-    for (int k = 0; k < K; k++) z[q][k] = 0.0;
-  moments_walk<K, NE>(st.flux, mod, st.xb, lo, split, 2 * min(g0, nb), min(2 * min(g1, nb), bb), lane, z);
-  moments_walk<K, NE>(st.flux, mod, st.xa, split, hi, 2 * max(g0 - nb, 0), min(2 * max(g1 - nb, 0), ba), lane, z);
-#pragma unroll
-  for (int q = 0; q < NE; q++) {
-    t[q] = warp_sum_vec<K>(z[q], lane);
-    if (!__all_sync(0xffffffffu, isfinite(t[q]))) {
-      double zz[K];
-#pragma unroll
-      for (int k = 0; k < K; k++) zz[k] = 0.0;
-      const int i0 = g0 < nb ? lo + 2 * PER * g0 : split + 2 * PER * (g0 - nb);
-      const int i1 = g1 < nb ? lo + 2 * PER * g1 : g1 == nb ? split : min(hi, split + 2 * PER * (g1 - nb));
-#pragma unroll 1
-      for (int i = i0 + lane; i < i1; i += 32) {
-        const float y = __fdividef(st.flux[i], mod[q][i]);
-        float Pk[K];
-        legendre<K>(i < split ? st.xb[i] : st.xa[i], Pk);
-#pragma unroll
-        for (int k = 0; k < K; k++) zz[k] += (double)(Pk[k] * y);
-      }
-      t[q] = warp_sum_vec<K>(zz, lane);
-    }
-  }
+    if (!__all_sync(0xffffffffu, isfinite(t[q]))) t[q] = chunk_moments_again<K>(st, mod[q], c, p, t[q]);
 }
 
 // Monomial coefficients of the Legendre polynomials, T[k][j] = coefficient
@@ -305,7 +358,7 @@ __device__ __forceinline__ float2 horner2(const float (&a)[K], float2 x) {
 // j1) of [a0, a1) to acc, p = the current chunk's polynomial, or (BLEND) pv
 // fac + cu (1 - fac) of the previous and the current chunk, for NE models of
 // one star.  ncc, ncp: the negated coefficients.
-template <int K, int NE, bool BLEND>
+template <int K, int NE, bool BLEND, bool DIV>
 __device__ __forceinline__ void resid_walk(const DevStar &st, const float *const (&mod)[NE], int a0, int a1, int j0, int j1,
                                            int lane, const float (&ncc)[NE][K], const float (&ncp)[NE][K],
                                            double (&acc)[NE]) {
@@ -316,7 +369,8 @@ __device__ __forceinline__ void resid_walk(const DevStar &st, const float *const
     for (int n = 0; n < NE; n++) part[n] = dup2(0.0f);
 #pragma unroll
     for (int u0 = 0; u0 < CU; u0 += N) {
-      float2 fl[N], md[NE][N], vr[N], xa[N], xb[N], fc[N];
+      float2 fl[N], md[NE][N], vr[N], xa[N];
+      [[maybe_unused]] float2 xb[N], fc[N];
 #pragma unroll
       for (int u = 0; u < N; u++) {
         fl[u] = ld(st.flux, u0 + u);
@@ -331,7 +385,7 @@ __device__ __forceinline__ void resid_walk(const DevStar &st, const float *const
       }
 #pragma unroll
       for (int u = 0; u < N; u++) {
-        const float2 iv = ld.mask(rcp2(vr[u]), u0 + u);
+        [[maybe_unused]] const float2 iv = DIV ? vr[u] : ld.mask(rcp2(vr[u]), u0 + u);
 #pragma unroll
         for (int n = 0; n < NE; n++) {
           float2 np;  // minus the continuum
@@ -342,7 +396,8 @@ __device__ __forceinline__ void resid_walk(const DevStar &st, const float *const
             np = horner2<K>(ncc[n], xa[u]);
           }
           const float2 r = __ffma2_rn(np, md[n][u], fl[u]);
-          part[n] = __ffma2_rn(ld.mask(__fmul2_rn(r, r), u0 + u), iv, part[n]);
+          if constexpr (DIV) part[n] = __fadd2_rn(ld.mask(div2(__fmul2_rn(r, r), iv), u0 + u), part[n]);
+          else part[n] = __ffma2_rn(ld.mask(__fmul2_rn(r, r), u0 + u), iv, part[n]);
         }
       }
     }
@@ -357,42 +412,67 @@ __device__ __forceinline__ double warp_sum_all(double v) {
   return v;
 }
 
-// chi2 of piece p of chunk section c (continuum_fitting.rs:280-360) by one
-// warp for NE models, the sums on every lane: chunk 0 alone on [50, start_1);
-// chunk c >= 1 blended with chunk c - 1 (sin^2 factor) on [start_c,
-// stop_{c-1}), then alone up to start_{c+1} (N - 50 for the last).
-template <int K, int NE>
-__device__ __forceinline__ void chunk_resid(const DevStar &st, const float *const (&mod)[NE], int c, int p, int lane,
-                                            const float (&ncc)[NE][K], const float (&ncp)[NE][K], double (&t)[NE]) {
-  constexpr int PB = 64, PA = 32 * chunk_cu<K>();  // pixels per block: blended, alone
-  const int nc = st.n_chunks;
-  const int s0 = c == 0 ? 50 : st.cstart[c], sp = c == 0 ? 50 : st.cstop[c - 1];
-  const int nx = c == nc - 1 ? st.n_obs - 50 : st.cstart[c + 1];
-  const int bb = blocks_of(s0, sp, PB), ba = blocks_of(sp, nx, PA), nb = (bb + 1) / 2, na = (ba + 1) / 2;
-  const int b0 = nb * p / CHUNK_PIECES, b1 = nb * (p + 1) / CHUNK_PIECES;
-  const int g0 = na * p / CHUNK_PIECES, g1 = na * (p + 1) / CHUNK_PIECES;
-  double acc[NE];
-#pragma unroll
-  for (int n = 0; n < NE; n++) acc[n] = 0.0;
-  resid_walk<K, NE, true>(st, mod, s0, sp, 2 * b0, min(2 * b1, bb), lane, ncc, ncp, acc);
-  resid_walk<K, NE, false>(st, mod, sp, nx, 2 * g0, min(2 * g1, ba), lane, ncc, ncp, acc);
-#pragma unroll
-  for (int n = 0; n < NE; n++) {
-    t[n] = warp_sum_all(acc[n]);
-    if (!isfinite(t[n])) {
-      double a = 0.0;
-      auto add = [&](int i, float np) {
-        const float r = fmaf(np, mod[n][i], st.flux[i]);
-        a += (double)__fdividef(r * r, st.var[i]);
-      };
-#pragma unroll 1
-      for (int i = s0 + 2 * PB * b0 + lane; i < min(sp, s0 + 2 * PB * b1); i += 32)
-        add(i, horner2<K>(ncp[n], dup2(st.xa[i])).x * st.fac[i] + horner2<K>(ncc[n], dup2(st.xb[i])).x * (1.0f - st.fac[i]));
-#pragma unroll 1
-      for (int i = sp + 2 * PA * g0 + lane; i < min(nx, sp + 2 * PA * g1); i += 32) add(i, horner2<K>(ncc[n], dup2(st.xa[i])).x);
-      t[n] = warp_sum_all(a);
-    }
+// Piece p of chunk section c (continuum_fitting.rs:280-360): chunk 0 alone on
+// [50, start_1); chunk c >= 1 blended with chunk c - 1 (sin^2 factor) on
+// [start_c, stop_{c-1}), then alone up to start_{c+1} (N - 50 for the last).
+template <int K>
+struct ResidPiece {
+  static constexpr int PB = 64, PA = 32 * chunk_cu<K>();  // pixels per block: blended, alone
+  int s0, sp, nx, bb, ba, b0, b1, g0, g1;
+  __device__ __forceinline__ ResidPiece(const DevStar &st, int c, int p) {
+    s0 = c == 0 ? 50 : st.cstart[c];
+    sp = c == 0 ? 50 : st.cstop[c - 1];
+    nx = c == st.n_chunks - 1 ? st.n_obs - 50 : st.cstart[c + 1];
+    bb = blocks_of(s0, sp, PB);
+    ba = blocks_of(sp, nx, PA);
+    const int nb = (bb + 1) / 2, na = (ba + 1) / 2;
+    b0 = nb * p / CHUNK_PIECES;
+    b1 = nb * (p + 1) / CHUNK_PIECES;
+    g0 = na * p / CHUNK_PIECES;
+    g1 = na * (p + 1) / CHUNK_PIECES;
   }
+  template <int NE, bool DIV>
+  __device__ __forceinline__ void sums(const DevStar &st, const float *const (&mod)[NE], int lane,
+                                       const float (&ncc)[NE][K], const float (&ncp)[NE][K], double (&t)[NE]) const {
+    double acc[NE];
+#pragma unroll
+    for (int n = 0; n < NE; n++) acc[n] = 0.0;
+    resid_walk<K, NE, true, DIV>(st, mod, s0, sp, 2 * b0, min(2 * b1, bb), lane, ncc, ncp, acc);
+    resid_walk<K, NE, false, DIV>(st, mod, sp, nx, 2 * g0, min(2 * g1, ba), lane, ncc, ncp, acc);
+#pragma unroll
+    for (int n = 0; n < NE; n++) t[n] = warp_sum_all(acc[n]);
+  }
+};
+
+// the negated coefficients of section c and of the one before, of NE evaluations
+template <int K, int NE>
+__device__ __forceinline__ void section_coefs(const float (*cfs)[K], int nc, int c, float (&ncc)[NE][K], float (&ncp)[NE][K]) {
+#pragma unroll
+  for (int n = 0; n < NE; n++)
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      ncc[n][k] = -cfs[n * nc + c][k];
+      ncp[n][k] = c > 0 ? -cfs[n * nc + c - 1][k] : 0.0f;
+    }
+}
+
+// The sum of one evaluation over a piece, formed with divisions: of a faint
+// star, or where the sum t came out infinite or NaN and a variance is that
+// small.  Not inlined (see chunk_moments_again).
+template <int K>
+__device__ __noinline__ double chunk_resid_div(const DevStar &st, const float *model, int c, int p, const float (*cfs)[K],
+                                               bool faint, double t) {
+  const int lane = threadIdx.x & 31;
+  const ResidPiece<K> P(st, c, p);
+  if (!faint && !any_subnormal(st.var, P.s0 + 2 * P.PB * P.b0, min(P.sp, P.s0 + 2 * P.PB * P.b1), lane) &&
+      !any_subnormal(st.var, P.sp + 2 * P.PA * P.g0, min(P.nx, P.sp + 2 * P.PA * P.g1), lane))
+    return t;
+  float ncc[1][K], ncp[1][K];
+  section_coefs<K, 1>(cfs, 0, c, ncc, ncp);
+  const float *const mod[1] = {model};
+  double s[1];
+  P.template sums<1, true>(st, mod, lane, ncc, ncp, s);
+  return s[0];
 }
 
 // whether evaluation e is one for k_chunk_fit<K> to fit; one that failed
@@ -412,12 +492,13 @@ __device__ __forceinline__ bool chunk_eval(const EvalBatch &b, const DevStar &st
 // NE evaluations e, e + 1, ... of one star by the CTA
 template <int K, int NE, int NW>
 __device__ __forceinline__ void chunk_fit(const EvalBatch &b, const DevStar &st, int e, double (*zs)[K], float (*cfs)[K],
-                                          double *part) {
+                                          double *part, int *faint) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float *mod[NE];
 #pragma unroll
   for (int n = 0; n < NE; n++) mod[n] = model_row(b, b.prep[e + n], e + n);
   const int nc = st.n_chunks, items = nc * CHUNK_PIECES, slot = chunk_slot<K>(lane);
+  const bool sample = faint_star(st);
   for (int it = warp; it < items; it += NW) {
     double z[NE];
     chunk_moments<K, NE>(st, mod, it / CHUNK_PIECES, it % CHUNK_PIECES, lane, z);
@@ -425,7 +506,8 @@ __device__ __forceinline__ void chunk_fit(const EvalBatch &b, const DevStar &st,
     for (int n = 0; n < NE; n++)
       if (slot < K) zs[n * items + it][slot] = z[n];  // the lanes of a slot hold the same sum
   }
-  __syncthreads();
+  const int f = __syncthreads_or(sample);
+  if (threadIdx.x == 0) *faint = f;  // kept out of the registers of the walks
   // (evaluation, chunk) pairs spread over the warps
   for (int i = lane * NW + warp; i < NE * nc; i += 32 * NW) {
     double *a = zs[i * CHUNK_PIECES];
@@ -434,21 +516,27 @@ __device__ __forceinline__ void chunk_fit(const EvalBatch &b, const DevStar &st,
     chunk_coefs<K>(b, st, e + i / nc, i % nc, a, cfs[i]);
   }
   __syncthreads();
-  for (int it = warp; it < items; it += NW) {
-    const int c = it / CHUNK_PIECES;
-    float ncc[NE][K], ncp[NE][K];
-#pragma unroll
-    for (int n = 0; n < NE; n++)
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        ncc[n][k] = -cfs[n * nc + c][k];
-        ncp[n][k] = c > 0 ? -cfs[n * nc + c - 1][k] : 0.0f;
+  if (*reinterpret_cast<volatile int *>(faint)) {
+    for (int i = warp; i < NE * items; i += NW) {
+      const int n = i / items, it = i % items;
+      const double t = chunk_resid_div<K>(st, NE > 1 && n ? mod[NE - 1] : mod[0], it / CHUNK_PIECES, it % CHUNK_PIECES, cfs + n * nc, true, 0.0);
+      if (lane == 0) part[i] = t;
+    }
+  } else {
+    for (int it = warp; it < items; it += NW) {
+      const int c = it / CHUNK_PIECES, p = it % CHUNK_PIECES;
+      double t[NE];
+      {
+        float ncc[NE][K], ncp[NE][K];
+        section_coefs<K, NE>(cfs, nc, c, ncc, ncp);
+        ResidPiece<K>(st, c, p).template sums<NE, false>(st, mod, lane, ncc, ncp, t);
       }
-    double t[NE];
-    chunk_resid<K, NE>(st, mod, c, it % CHUNK_PIECES, lane, ncc, ncp, t);
 #pragma unroll
-    for (int n = 0; n < NE; n++)
-      if (lane == 0) part[n * items + it] = t[n];
+      for (int n = 0; n < NE; n++) {
+        if (!isfinite(t[n])) t[n] = chunk_resid_div<K>(st, mod[n], c, p, cfs + n * nc, false, t[n]);
+        if (lane == 0) part[n * items + it] = t[n];
+      }
+    }
   }
   __syncthreads();
   if (threadIdx.x < NE) {
@@ -473,20 +561,21 @@ __global__ void __launch_bounds__(32 * NW, NW > 8 ? 1 : chunk_ctas(K, NE)) k_chu
   __shared__ double zs[NE * MAX_CHUNKS * CHUNK_PIECES][K];
   __shared__ float cfs[NE * MAX_CHUNKS][K];
   __shared__ double part[NE * MAX_CHUNKS * CHUNK_PIECES];
+  __shared__ int faint;
   const int e0 = blockIdx.x * NE, n = min(NE, b.E - e0);
   bool mine[NE];
 #pragma unroll
   for (int q = 0; q < NE; q++) mine[q] = q < n && chunk_eval<K>(b, b.stars[b.prep[e0 + q].star], e0 + q);
   if constexpr (NE == 2) {
     if (mine[0] && mine[1] && b.prep[e0].star == b.prep[e0 + 1].star) {
-      chunk_fit<K, 2, NW>(b, b.stars[b.prep[e0].star], e0, zs, cfs, part);
+      chunk_fit<K, 2, NW>(b, b.stars[b.prep[e0].star], e0, zs, cfs, part, &faint);
       return;
     }
   }
 #pragma unroll 1
   for (int q = 0; q < n; q++) {
     if (!(q == 0 ? mine[0] : mine[NE - 1])) continue;
-    chunk_fit<K, 1, NW>(b, b.stars[b.prep[e0 + q].star], e0 + q, zs, cfs, part);
+    chunk_fit<K, 1, NW>(b, b.stars[b.prep[e0 + q].star], e0 + q, zs, cfs, part, &faint);
     __syncthreads();
   }
 }
