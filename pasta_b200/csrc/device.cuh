@@ -35,17 +35,6 @@ __device__ __forceinline__ GridGeom geom_shared(const GridGeom &g, double *buf) 
   return r;
 }
 
-// Bulk prefetch of floats [lo, hi) of a row into L2 (one instruction, issued
-// by one thread; a hint, nothing waits for it).  The row must start on a
-// 16-byte boundary and hold hi rounded up to 4 floats.
-__device__ __forceinline__ void prefetch_row_l2(const float *row, int lo, int hi) {
-  lo &= ~3;
-  hi = (hi + 3) & ~3;
-  if (hi <= lo) return;
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(row + lo), "r"((unsigned)(hi - lo) * 4u)
-               : "memory");
-}
-
 // model at the observed pixels of evaluation e
 __device__ __forceinline__ const float *model_row(const EvalBatch &b, const EvalPrep &P, int e) {
   if (b.given) return b.given + (size_t)e * b.given_stride;
@@ -82,17 +71,10 @@ struct Resampler {
       else if (k == N) idx = (double)N - 1.0;
       else idx = __dadd_rn(__dadd_rn(__ddiv_rn(wl - wl_vals[k - 1], wl_vals[k] - wl_vals[k - 1]), (double)k), -1.0);
     }
-    return from_index(idx);
-  }
-  __device__ __forceinline__ ResPos from_index(double idx) const {
     const double fl = floor(idx);
     int j = fl > 0 ? (int)fl : 0;
     if (j > N - 2) j = N - 2;  // the preparation kernel rejected j + 1 >= N already
     return ResPos{j, (float)idx - (float)j};
-  }
-  // position from an already loaded float index (uniform grids)
-  __device__ __forceinline__ ResPos pos_from_fidx(double fx) const {
-    return from_index(kind == WL_LOG ? fx + shift_log : __dadd_rn(__dmul_rn(shift_factor, fx), lin_offset));
   }
   __device__ __forceinline__ float operator()(int i) const {
     if (given) return given[i];
