@@ -1494,6 +1494,7 @@ void tune_direct(pasta_grid *g) {
   dl.alloc((size_t)E * 5);
   DBuf<int> de;
   de.upload(std::vector<int>(E, 0));
+  wait_uploads();
   ensure_workspace(g, E, 0);
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
@@ -1595,6 +1596,7 @@ void tune_interp_tc(pasta_grid *g) {
   dl.alloc((size_t)E * 5);
   DBuf<int> de;
   de.upload(std::vector<int>(E, 0));
+  wait_uploads();
   ensure_workspace(g, E, 0);
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
@@ -1756,6 +1758,7 @@ int pasta_grid_create(const double *labels, const uint16_t *spectra, const float
     if (wl_kind == WL_LIN) d.dvelo = wl_b / ((wl_a + wl_a + wl_b * (double)n_px) / 2.0);
     else if (wl_kind == WL_LOG) d.dvelo = M_LN10 * wl_b;
     else d.dvelo = 0.0;
+    wait_uploads();
     tune_direct(g.get());
     tune_interp_tc(g.get());
     *out = g.release();
@@ -1927,6 +1930,7 @@ int pasta_dispersion_create(int synth_kind, double synth_a, double synth_b, int6
     d->dwl.upload(d->wl);
     if (!d->gk.empty()) d->dgk.upload(d->gk);
     if (d->dev_kind == DISP_FIXED) d->dgspec.upload(kernel_spectrum(d->gk));
+    wait_uploads();
     *out = d.release();
   });
 }
@@ -1974,6 +1978,7 @@ int pasta_continuum_create(int kind, const double *wl, int64_t n, int n_chunks, 
     } else if (kind != PASTA_CONT_CONSTANT) {
       fail(PASTA_E_ARG, "invalid continuum kind %d", kind);
     }
+    wait_uploads();
     *out = c.release();
   });
 }
@@ -3254,6 +3259,7 @@ void server_rebuild(pasta_server *sv, int Pmax) {
   sv->pp.assign(sv->slots, PsoParams{});
   sv->W.params.upload(sv->pp);
   sv->dstars.upload(sv->hstars);
+  wait_uploads();
   if (sv->exec) { cudaGraphExecDestroy(sv->exec); sv->exec = nullptr; }
   if (sv->graph) { cudaGraphDestroy(sv->graph); sv->graph = nullptr; }
 }

@@ -61,13 +61,13 @@ int scratch_device();
 cudaStream_t scratch_stream();
 void scratch_flush(int dev);
 
-// Copies a host array to the device and waits for it.  cudaMemcpy returns when
-// a pageable source has been staged, and what it still has under way is on the
-// legacy stream, which the library's non-blocking streams do not wait for.
-inline void copy_to_device(void *dst, const void *src, size_t n) {
-  CK(cudaMemcpy(dst, src, n, cudaMemcpyHostToDevice));
-  CK(cudaStreamSynchronize(cudaStreamLegacy));
-}
+// Waits for the DBuf uploads made so far.  cudaMemcpy returns when a pageable
+// source has been staged, and what it still has under way is on the legacy
+// stream, which the library's non-blocking streams do not wait for: whoever
+// makes an object waits once, before it hands it out or enqueues work on it
+// (a wait after every upload keeps the next one from being staged meanwhile: a
+// chunk continuum of 60,000 pixels 2.45 ms instead of 2.0).
+inline void wait_uploads() { CK(cudaStreamSynchronize(cudaStreamLegacy)); }
 
 // POOL: scratch of one call or fit (see scratch_take); its uploads are ordered
 // on the device's stream
@@ -119,7 +119,7 @@ struct DBuf {
     alloc(count);
     if (!count) return;
     if (POOL) CK(cudaMemcpyAsync(p, h, count * sizeof(T), cudaMemcpyHostToDevice, scratch_stream()));
-    else copy_to_device(p, h, count * sizeof(T));
+    else CK(cudaMemcpy(p, h, count * sizeof(T), cudaMemcpyHostToDevice));  // see wait_uploads
   }
   void upload(const std::vector<T> &v) { upload(v.data(), v.size()); }
 };
@@ -243,7 +243,8 @@ Ctx &ctx() {
       t[k] = make_float2((float)std::cos(a), (float)std::sin(a));
     }
     c->tw.alloc(t.size(), false);
-    copy_to_device(c->tw.p, t.data(), t.size() * sizeof(float2));
+    CK(cudaMemcpy(c->tw.p, t.data(), t.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    wait_uploads();
     slot = std::move(c);
   }
   CK(cudaSetDevice(slot->dev));

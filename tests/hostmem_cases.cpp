@@ -312,13 +312,14 @@ static void captures_are_alone() {
   cap.finish(&g);
 }
 
-// Uploads are complete when they return: nothing orders the library's streams
-// behind the legacy stream.
+// A context's own table is complete when it is handed out, other uploads after
+// wait_uploads(): nothing orders the library's streams behind the legacy stream.
 static void uploads_are_waited_for() {
   ctx();
   EXPECT(fake::legacy_pending == 0);
   DBuf<int> a;
   a.upload(std::vector<int>(1000, 3));
+  wait_uploads();
   EXPECT(fake::legacy_pending == 0 && a.p[999] == 3);
 }
 
