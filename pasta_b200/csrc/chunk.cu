@@ -61,7 +61,7 @@ __device__ __forceinline__ float poly_eval(const float *coef, float x) {
 // its arrays and the Legendre values, and the blocks of a chunk are spread
 // over CHUNK_PIECES warps, so that spectra with fewer chunks than warps keep
 // all warps busy.  4,000 evaluations of 60,000 pixels, degree 5 (ncu): 654 M
-// warp instructions and 914 us with one pixel per operation, 245 M and 677 us
+// warp instructions and 914 us with one pixel per operation, 250 M and 655 us
 // now; 40 evaluations of 15,000 pixels, degree 8: 53 -> 31 us.
 constexpr int CHUNK_PIECES = 4;
 // pixels of a lane in a block: 8 up to degree 5, 4 above
@@ -584,7 +584,7 @@ template <int K>
 static void launch_chunk(const EvalBatch &b, cudaStream_t s) {
   // Pairs share their star's reads once they fill the GPU (two CTAs per SM).
   // Above degree 7 their sums do not fit the registers.  4,000 evaluations of
-  // 60,000 pixels, degree 5: 814 us alone, 677 us in pairs.
+  // 60,000 pixels, degree 5: 814 us alone, 677 us in pairs (655 us now).
   if constexpr (K <= 8) {
     if (b.seg_len != 1 && b.E >= 4 * num_sms()) {
       k_chunk_fit<K, 2, 8><<<(b.E + 1) / 2, 256, 0, s>>>(b);

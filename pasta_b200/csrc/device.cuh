@@ -116,9 +116,9 @@ __device__ __forceinline__ float instrument(const DevStar &st, int N, int i, int
   } else {
     if (i < h || i >= N - h) return r(i);
     // tap-major: the lanes of a warp work neighbouring pixels and read
-    // neighbouring words (pixel-major taps, a stride of w words between the
-    // lanes, made k_broaden 1.51 ms for 1,000 evaluations of 80,000 pixels
-    // and 17 taps, against 1.27 ms with this loop)
+    // neighbouring words (k_broaden, when it had this loop too: 1.51 ms for
+    // 1,000 evaluations of 80,000 pixels and 17 taps with pixel-major taps, a
+    // stride of w words between the lanes, 1.27 ms with these)
     const float *kk = st.gk + i;
     for (int t = 0; t < w; t++) acc = fmaf(__ldg(&kk[(size_t)t * N]), r(i - h + t), acc);
   }

@@ -1646,7 +1646,10 @@ void tune_interp_tc(pasta_grid *g) {
       fprintf(stderr, "pasta_b200 tune: %lld px, groups of %d: CUDA cores %.4f ms, tensor cores %.4f ms\n",
               (long long)g->npx, gs, tm[0], tm[1]);
     // the first size that gains a sixth: at a near-tie the choice would vary
-    // from one process to the next, and the two forms round differently
+    // from one process to the next, and the two forms round differently (a
+    // sixth is more than that takes; it leaves the thresholds at 32, 8 and 8
+    // members for 80,000, 20,000 and 120,000 pixels, where a plain win had
+    // them before both forms became faster)
     if (tm[1] < tm[0]) {
       if (best > SEG && tm[1] < (5.0f / 6.0f) * tm[0]) best = gs;
     } else {

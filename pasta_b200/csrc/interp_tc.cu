@@ -25,9 +25,9 @@
 //               loads of four 128-pixel rows each, from the grid resident in
 //               this GPU's own memory, each CTA loading for itself) into a ring of NSTG staging
 //               buffers;
-//   warp 1      one thread issues the 24 tcgen05.mma of a tile (kind::f16,
-//               M = 128, N = members rounded up to 16) into one of ND
-//               tensor-memory accumulators;
+//   warp 1      the whole warp follows the tiles and its elected lane issues
+//               the 24 tcgen05.mma of each (kind::f16, M = 128, N = members
+//               rounded up to 16) into one of ND tensor-memory accumulators;
 //   warps 2-9   converters: staging -> the bf16 byte planes of A (a ring of
 //               NA buffers in tensor memory), and each item's B (two buffers, so the next
 //               item's weights are written while the last tiles of the

@@ -408,7 +408,7 @@ __device__ __forceinline__ void rec_load(GroupRec *dst, const GroupRec *src) {
 }
 
 // Grid: x = segment, y = tile of IT_TILE pixels, so CTAs that run together read
-// the same tile slab of the resident grid (57 MB for 13,860 x 80,000), which
+// the same tile slab of the resident grid (28 MB for 13,860 models), which
 // stays in L2; z = slice of the segment's groups (groups z, z + Z, ...), more
 // than one only for batches too small to fill the GPU otherwise.  Groups have
 // disjoint members, so the slicing does not change any result.  The next
